@@ -1,5 +1,5 @@
-// EXACT-mode sweeps: one i-particle per thread, j-particles streamed through
-// shared memory in tiles and summed in source order.  With the pair
+// EXACT-mode sweeps: the terms of the pairs are formed in parallel over i
+// and j and added to each i's sums in source order.  With the pair
 // arithmetic of tg_pairs.cuh and this file compiled with -fmad=false, every
 // output is bit-identical to the reference C kernel (tupan/lib/src/*.c) on
 // the same inputs, for REAL = double and REAL = float.
@@ -18,41 +18,93 @@ namespace tg {
 constexpr int EXACT_THREADS = 128;
 constexpr int EXACT_TILE = 128;
 
-template <class Op, typename R>
-__global__ void __launch_bounds__(EXACT_THREADS)
-exact_sweep(const Sweep s)
+// The pair terms of a tile, I = 2^li particles i (a block's) against
+// J = T P / I consecutive j, P pairs (P i's, one j) a thread; the terms go
+// through shared memory to the I x NO threads that hold the sums and fold
+// them in j order.  Double buffered: one barrier a tile, a warp that holds
+// no sum goes on to the next tile's pairs.
+//
+// Why: a sum's additions have to stay in order, the terms need not.  One i a
+// thread over all j (the form this replaces) put a 256-body sweep on two SMs
+// and a 3001-body one on 24, each at the latency of a chain of whole pairs;
+// here only the additions are a chain (64 cycles each in double) and any ni
+// fills the chip.  Bound: the FP64 pipe (20 additions of 19 SM cycles a
+// warp of AccJerk pairs; ncu at N = 8192: 71 % of its peak, the integer pipe
+// that carries the products 57 %).  No j prefetch and 64 registers (eight
+// blocks of 128 an SM) beat a prefetch at four blocks by 10 %: the chains of
+// dependent additions want warps.  Measured, double, Phi / AccJerk /
+// SnapCrackle / Tstep: N = 256 268 / 533 / 1216 / 687 us before, 17 / 19 /
+// 27 / 25 us now; N = 3001 2.98 / 6.09 / 14.1 / 7.70 ms, now 0.32 / 0.55 /
+// 1.41 / 0.65 ms; N = 32768 61 / 128 / 302 / 157 ms, now 21 / 51 / 141 /
+// 54 ms.  float takes four i a thread (one load of a j for four pairs, one
+// 16-byte store of a term): Phi + Acc at N = 10007 2.3 ms before, 0.62 ms.
+template <class Op, typename R, int T, int P, int BLK>
+__global__ void __launch_bounds__(T, BLK)
+exact_terms(const Sweep s, const int li)
 {
-    constexpr int NA = Op::NA;
-    __shared__ R tile[NA][EXACT_TILE];
+    constexpr int NA = Op::NA, NO = Op::NO;
+    constexpr int LP = P == 1 ? 0 : P == 2 ? 1 : 2;
+    static_assert(P == 1 << LP, "P is 1, 2 or 4");
+    __shared__ __align__(16) R buf[2][NO][T * P];
     const uint64_t ni = s.ni_dev ? (uint64_t)*s.ni_dev : s.ni, nj = s.nj;
+    const uint64_t i0 = (uint64_t)blockIdx.x << li;
     // blocks past a device-side count have no i (the whole block leaves)
-    if ((uint64_t)blockIdx.x * EXACT_THREADS >= ni) return;
-    const uint64_t i = (uint64_t)blockIdx.x * EXACT_THREADS + threadIdx.x;
-    const uint64_t ic = i < ni ? i : ni - 1;
-    R ip[NA];
+    if (i0 >= ni) return;
+    const int tid = threadIdx.x;
+    const int g = tid & ((1 << (li - LP)) - 1), row = tid >> (li - LP);
+    const int J = T * P >> li;
+    const int c = tid >> li, ii = tid & ((1 << li) - 1);
+    const bool sums = c < NO;
+    R o = R(0);
+    if (nj) {
+        R ip[P][NA], jp[NA];
 #pragma unroll
-    for (int a = 0; a < NA; ++a) ip[a] = ((const R *)s.ip[a])[ic];
-    R o[Op::NO];
-    Op::init(o);
-    for (uint64_t j0 = 0; j0 < nj; j0 += EXACT_TILE) {
-        const int n = (int)((nj - j0) < EXACT_TILE ? (nj - j0) : EXACT_TILE);
-        __syncthreads();
-        for (int t = threadIdx.x; t < NA * EXACT_TILE; t += EXACT_THREADS) {
-            const int a = t / EXACT_TILE, jj = t % EXACT_TILE;
-            if (jj < n) tile[a][jj] = ((const R *)s.jp[a])[j0 + jj];
+        for (int p = 0; p < P; ++p) {
+            const uint64_t i = i0 + g * P + p < ni ? i0 + g * P + p : ni - 1;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) ip[p][a] = ((const R *)s.ip[a])[i];
         }
-        __syncthreads();
-        for (int jj = 0; jj < n; ++jj) {
-            R jp[NA];
+        Softening<R> soft2[P];
 #pragma unroll
-            for (int a = 0; a < NA; ++a) jp[a] = tile[a][jj];
-            Op::pair(ip, jp, o, s);
+        for (int p = 0; p < P; ++p)
+            soft2[p].set(ip[p][4], ((const R *)s.jp[4])[0]);
+        int b = 0;
+        for (uint64_t j0 = 0; j0 < nj; j0 += J, b ^= 1) {
+            const uint64_t j = j0 + row < nj ? j0 + row : nj - 1;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) jp[a] = ((const R *)s.jp[a])[j];
+            R t[NO][P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                R tp[NO];
+                Op::terms(ip[p], jp, tp, s, soft2[p]);
+#pragma unroll
+                for (int k = 0; k < NO; ++k) t[k][p] = tp[k];
+            }
+#pragma unroll
+            for (int k = 0; k < NO; ++k) {
+                R *w = &buf[b][k][tid * P];
+                if constexpr (P == 4)
+                    *(float4 *)w = make_float4(t[k][0], t[k][1], t[k][2],
+                                               t[k][3]);
+                else
+#pragma unroll
+                    for (int p = 0; p < P; ++p) w[p] = t[k][p];
+            }
+            __syncthreads();
+            if (sums) {
+                const int n = nj - j0 < (uint64_t)J ? (int)(nj - j0) : J;
+                const R *q = &buf[b][c][ii];
+#pragma unroll 8
+                for (int k = 0; k < n; ++k) o = Op::fold(c, o, q[k << li]);
+            }
         }
     }
-    if (i < ni) {
-        Op::finish(ip, o, s);
+    if (sums && i0 + ii < ni) {
+        R ip[NA];
 #pragma unroll
-        for (int c = 0; c < Op::NO; ++c) ((R *)s.out[c])[i] = o[c];
+        for (int a = 0; a < NA; ++a) ip[a] = ((const R *)s.ip[a])[i0 + ii];
+        ((R *)s.out[c])[i0 + ii] = Op::finish(c, ip, o, s);
     }
 }
 
@@ -128,8 +180,18 @@ __global__ void exact_kepler(const Sweep s, long long budget, unsigned *err)
 template <class Op, typename R>
 static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
 {
-    const unsigned blocks = (unsigned)((s.ni + EXACT_THREADS - 1) / EXACT_THREADS);
-    exact_sweep<Op, R><<<blocks, EXACT_THREADS, 0, st>>>(s);
+    constexpr int T = EXACT_THREADS;
+    constexpr int P = sizeof(R) == 8 ? 1 : Op::WIDE ? 1 : 4;
+    constexpr int BLK = sizeof(R) == 8 ? (Op::WIDE ? 4 : 8) : 6;
+    // As many i a block as leave 600 blocks (four an SM): more i share a j
+    // load and fill the warps that add, fewer leave SMs idle (AccJerk at
+    // N = 3001: 751 blocks of 4 i 0.55 ms, 376 of 8 i 0.70 ms; at 32768
+    // 8 or 16 i within 1 %).  The I x NO sums have to fit the block.
+    int li = 5;
+    while ((Op::NO << li) > T) --li;
+    while ((1 << li) > P && (s.ni >> li) < 600) --li;
+    const unsigned blocks = (unsigned)((s.ni + (1u << li) - 1) >> li);
+    exact_terms<Op, R, T, P, BLK><<<blocks, T, 0, st>>>(s, li);
     g_launch_count += 1;
     return cudaGetLastError();
 }

@@ -314,15 +314,18 @@ __device__ void sub_sweep(SubState &S, int ilo, int ni, int jlo, int nj,
         double ip[Op::NA], jp[Op::NA], o[Op::NO];
 #pragma unroll
         for (int a = 0; a < Op::NA; ++a) ip[a] = S.f[a][ilo + t];
-        Op::init(o);
+#pragma unroll
+        for (int c = 0; c < Op::NO; ++c) o[c] = 0.0;
+        Softening<double> soft2;
+        soft2.set(ip[4], S.f[F_E2][jlo]);
         for (int j = 0; j < nj; ++j) {
 #pragma unroll
             for (int a = 0; a < Op::NA; ++a) jp[a] = S.f[a][jlo + j];
-            Op::pair(ip, jp, o, sw);
+            fold_pair<Op>(ip, jp, o, sw, soft2);
         }
-        Op::finish(ip, o, sw);
 #pragma unroll
-        for (int c = 0; c < Op::NO; ++c) S.f[first_out + c][ilo + t] = o[c];
+        for (int c = 0; c < Op::NO; ++c)
+            S.f[first_out + c][ilo + t] = Op::finish(c, ip, o[c], sw);
     }
     __syncthreads();
 }

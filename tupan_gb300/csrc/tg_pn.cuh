@@ -229,21 +229,22 @@ __device__ PnTerm<R> pn7(R im, R jm, R im2, R jm2, R imjm, R inv_r, R inv_r2,
 template <typename R>
 struct PnAccPair {
     static constexpr int NA = 8, NO = 3;
-    __device__ static void init(R *o) { o[0] = o[1] = o[2] = R(0); }
-    __device__ static void pair(const R *ip, const R *jp, R *o,
-                                const Sweep &s)
+    static constexpr bool WIDE = true;    // keeps 128 registers a thread
+    __device__ __forceinline__ static void terms(const R *ip, const R *jp,
+                                                 R *t, const Sweep &s,
+                                                 Softening<R> &soft2)
     {
         const uint64_t order = (uint64_t)s.iscal;
         R im = ip[0], jm = jp[0];
         R ivx = ip[5], ivy = ip[6], ivz = ip[7];
         R jvx = jp[5], jvy = jp[6], jvz = jp[7];
         R dx = ip[1] - jp[1], dy = ip[2] - jp[2], dz = ip[3] - jp[3];
-        R h2 = ip[4] + jp[4];
+        R h2 = soft2.sum(ip[4], jp[4]);
         R ux = ivx - jvx, uy = ivy - jvy, uz = ivz - jvz;
         R r2 = dx * dx + dy * dy + dz * dz;
         R v2 = ux * ux + uy * uy + uz * uz;
-        R inv_r2 = masked_inv_r2(r2, h2);
-        R inv_r = sqrt(inv_r2);
+        R inv_r2, inv_r;
+        inv_root(r2, h2, &inv_r2, &inv_r);
         R inv_r3 = inv_r2 * inv_r;
 
         PnTerm<R> p2 = {0, 0}, p4 = {0, 0}, p5 = {0, 0}, p6 = {0, 0},
@@ -293,11 +294,12 @@ struct PnAccPair {
         pb += ((((((p7.b + p6.b) + p5.b) + p4.b) + p3.b) + p2.b) + p1.b);
         pa *= jm * inv_r3;
         pb *= jm * inv_r2;
-        o[0] += pa * dx + pb * ux;
-        o[1] += pa * dy + pb * uy;
-        o[2] += pa * dz + pb * uz;
+        t[0] = pa * dx + pb * ux;
+        t[1] = pa * dy + pb * uy;
+        t[2] = pa * dz + pb * uz;
     }
-    __device__ static void finish(const R *, R *, const Sweep &) {}
+    __device__ static R fold(int, R o, R t) { return o + t; }
+    __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
 };
 
 }  // namespace tg
