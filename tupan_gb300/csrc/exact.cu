@@ -16,7 +16,6 @@
 namespace tg {
 
 constexpr int EXACT_THREADS = 128;
-constexpr int EXACT_TILE = 128;
 
 // The pair terms of a tile, I = 2^li particles i (a block's) against
 // J = T P / I consecutive j, P pairs (P i's, one j) a thread; the terms go
@@ -110,49 +109,23 @@ exact_terms(const Sweep s, const int li)
 
 // sakura_kernel.c:33-62: Sigma_j (m_j/M)(two-body step - initial state).
 template <typename R>
-__global__ void __launch_bounds__(EXACT_THREADS)
-exact_sakura(const Sweep s, long long budget, unsigned *err)
-{
-    constexpr int NA = 8;
-    __shared__ R tile[NA][EXACT_TILE];
-    const uint64_t ni = s.ni, nj = s.nj;
-    const uint64_t i = (uint64_t)blockIdx.x * EXACT_THREADS + threadIdx.x;
-    const uint64_t ic = i < ni ? i : ni - 1;
-    const R dt = R(s.scal[0]);
-    const long long flag = s.iscal;
-    R ip[NA];
-#pragma unroll
-    for (int a = 0; a < NA; ++a) ip[a] = ((const R *)s.ip[a])[ic];
-    R o[6] = {0, 0, 0, 0, 0, 0};
-    bool exhausted = false;
-    for (uint64_t j0 = 0; j0 < nj; j0 += EXACT_TILE) {
-        const int n = (int)((nj - j0) < EXACT_TILE ? (nj - j0) : EXACT_TILE);
-        __syncthreads();
-        for (int t = threadIdx.x; t < NA * EXACT_TILE; t += EXACT_THREADS) {
-            const int a = t / EXACT_TILE, jj = t % EXACT_TILE;
-            if (jj < n) tile[a][jj] = ((const R *)s.jp[a])[j0 + jj];
-        }
-        __syncthreads();
-        for (int jj = 0; jj < n; ++jj) {
-            R jp[NA];
-#pragma unroll
-            for (int a = 0; a < NA; ++a) jp[a] = tile[a][jj];
-            R p0[6], p1[6], m, e2;
-            pair_state(ip, jp, p0, &m, &e2);
-            KepCtx<R> c = {0, budget, 0, false, false, R(0)};
-            evolve_pair(dt, flag, m, e2, p0, p1, c);
-            exhausted |= c.exhausted;
-            R mu = jp[0] / m;
-#pragma unroll
-            for (int q = 0; q < 6; ++q) o[q] += mu * (p1[q] - p0[q]);
-        }
+struct SakuraPair {
+    static constexpr int NA = 8, NO = 6;
+    static constexpr bool WIDE = true;
+    __device__ __forceinline__ static void terms(const R *ip, const R *jp,
+                                                 R *t, const Sweep &s,
+                                                 Softening<R> &)
+    {
+        R p0[6], p1[6], m, e2;
+        pair_state(ip, jp, p0, &m, &e2);
+        KepCtx<R> c = {0, s.budget, 0, false, false, R(0)};
+        evolve_pair(R(s.scal[0]), s.iscal, m, e2, p0, p1, c);
+        if (c.exhausted) atomicOr(s.err, (unsigned)DERR_KEPLER_BUDGET);
+        pair_term(jp[0], m, p0, p1, t);
     }
-    if (i < ni) {
-#pragma unroll
-        for (int q = 0; q < 6; ++q) ((R *)s.out[q])[i] = o[q];
-        if (exhausted) atomicOr(err, (unsigned)DERR_KEPLER_BUDGET);
-    }
-}
+    __device__ static R fold(int, R o, R t) { return o + t; }
+    __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
+};
 
 // kepler_solver_kernel.c:5-49 with kepler_solver_kernel_common.h:8-80: two
 // particles evolved in their centre-of-mass frame; outputs may alias inputs.
@@ -216,11 +189,10 @@ cudaError_t launch_exact(const Sweep &s, cudaStream_t st, long long budget,
     case K_NREG_X: return run_exact<NregXPair<R>, R>(s, st);
     case K_NREG_V: return run_exact<NregVPair<R>, R>(s, st);
     case K_SAKURA: {
-        const unsigned blocks =
-            (unsigned)((s.ni + EXACT_THREADS - 1) / EXACT_THREADS);
-        exact_sakura<R><<<blocks, EXACT_THREADS, 0, st>>>(s, budget, err);
-        g_launch_count += 1;
-        return cudaGetLastError();
+        Sweep k = s;
+        k.budget = budget;
+        k.err = err;
+        return run_exact<SakuraPair<R>, R>(k, st);
     }
     default: return cudaErrorInvalidValue;
     }

@@ -6,12 +6,13 @@
 // (r^2 > (64 m / v^2)^2, sakura_kernel_common.h:111-117), the rest the
 // iterative universal-variable solver.  Run inline, one Kepler pair stalls
 // its whole warp.  Here, for the flags the Sakura integrator uses (-1, +1):
-//   1. count, per i, the pairs that take the Kepler branch (cheap test);
-//   2. exclusive scan of the counts;
-//   3. sum the leapfrog pairs in j order and write the Kepler pairs' j
-//      indices, in j order, into each i's segment of a queue;
-//   4. solve the queue, one thread per pair (coherent work);
-//   5. add each i's Kepler contributions, in j order, to its leapfrog sum.
+//   1. sum the leapfrog pairs in j order, append the Kepler pairs (i, j and
+//      the rank among their i's) to a queue and count them per i;
+//   2. exclusive scan of the counts: pair (i, rank)'s place in j order;
+//   3. solve the queue, one thread per pair (coherent work);
+//   4. add each i's Kepler contributions, in j order, to its leapfrog sum.
+// The counts stay on the device; a queue that turns out too small is grown
+// and the sweep repeated.
 // The leapfrog branch is bit-identical to the reference (compiled without
 // contraction); the result differs from the reference's interleaved sum only
 // by the order of the additions, and the Kepler branch by CUDA's
@@ -202,7 +203,14 @@ k_pair_solve(const PairSolve P, unsigned *err)
 // Queued Sakura sweep (flags -1 and +1).
 // ---------------------------------------------------------------------------
 constexpr int SK_THREADS = 128;
-constexpr int SK_TILE = 128;
+
+// What a sweep reports back: Kepler pairs found, Laguerre-update histogram
+// (bin k: solves with k updates, the last 64 or more), error word.
+struct SakuraReport {
+    unsigned long long pairs;
+    unsigned long long hist[65];
+    unsigned err;
+};
 
 struct SakuraArgs {
     uint64_t ni, nj;
@@ -210,11 +218,13 @@ struct SakuraArgs {
     double *out[6];
     double dt;
     long long flag;
-    unsigned *cnt;          // ni (pass 1), then offsets (pass 2)
+    unsigned *cnt;          // ni counts (step 1), then offsets (step 2)
     unsigned *queue_j;      // Kepler pairs: j index
     unsigned *queue_i;      // Kepler pairs: i index
-    double *contrib;        // 6 per queued pair
-    int *iters;             // per queued pair (or null)
+    unsigned *queue_r;      // Kepler pairs: rank among their i's, in j order
+    unsigned long long cap; // queue entries
+    double *contrib;        // 6 per queued pair, in (i, j) order
+    SakuraReport *rep;
     long long budget;
     int use_mlp;
     int form;               // KeplerForm of the Kepler-branch solves
@@ -223,80 +233,110 @@ struct SakuraArgs {
 
 // Drift applied before the two-body step for flag -1 (sakura_kernel_common.h
 // :151-157); flag +1 evolves first and drifts after (:158-164).
-__device__ __forceinline__ bool sk_kepler(const double *ip, const double *jp,
-                                          double dt, long long flag,
-                                          double *p0, double *pre, double *m,
-                                          double *e2)
+__device__ __forceinline__ void sk_start(const double *ip, const double *jp,
+                                         double dt, long long flag,
+                                         double *p0, double *pre, double *m,
+                                         double *e2)
 {
     pair_state(ip, jp, p0, m, e2);
     for (int c = 0; c < 6; ++c) pre[c] = p0[c];
-    if (flag == -1) {
-        pre[0] -= pre[3] * dt;
-        pre[1] -= pre[4] * dt;
-        pre[2] -= pre[5] * dt;
-    }
-    return !takes_leapfrog(*m, pre);
+    if (flag == -1) pair_drift(pre, pre + 3, dt, true);
 }
 
-template <int PASS>
-__global__ void __launch_bounds__(SK_THREADS)
-k_sakura_pass(const SakuraArgs A)
+// Pairs in parallel over i and j, I = 2^li i a block, one pair a thread; the
+// leapfrog terms are folded in j order through shared memory (as
+// exact_terms does), the Kepler pairs of each i are queued in j order (their
+// terms enter the sum as +0, which changes no sum).
+//
+// One i a thread over all j, in two passes (count, then sum), the form this
+// replaces, ran a 4096-body sweep on 32 SMs with its quotients on the FP64
+// pipe: 23.9 ms a sweep with its solves, now 2.3 (N = 256: 1.70 ms, now
+// 0.18).  Bound: the FP64 pipe, 39 additions a pair at 19 SM cycles a warp
+// (1.3 ms of the 1.8 the kernel takes at N = 4096); eight blocks of 64
+// registers an SM beat five of 96 by 11 %.
+__global__ void __launch_bounds__(SK_THREADS, 8)
+k_sakura_pass(const SakuraArgs A, const int li)
 {
-    __shared__ double tile[8][SK_TILE];
-    const uint64_t i = (uint64_t)blockIdx.x * SK_THREADS + threadIdx.x;
-    const uint64_t ic = i < A.ni ? i : A.ni - 1;
+    constexpr int T = SK_THREADS, NO = 6;
+    __shared__ double buf[2][NO][T];
+    __shared__ unsigned near[2][T / 32];
+    const int tid = threadIdx.x, ii = tid & ((1 << li) - 1), row = tid >> li;
+    const int J = T >> li;
+    const uint64_t i0 = (uint64_t)blockIdx.x << li;
+    const uint64_t i = i0 + ii < A.ni ? i0 + ii : A.ni - 1;
     double ip[8];
-    for (int a = 0; a < 8; ++a) ip[a] = A.ip[a][ic];
+#pragma unroll
+    for (int a = 0; a < 8; ++a) ip[a] = A.ip[a][i];
     const double dt = A.dt;
     const long long flag = A.flag;
-    double o[6] = {0, 0, 0, 0, 0, 0};
+    const bool sums = row < NO, queues = row == NO && i0 + ii < A.ni;
+    double o = 0.0;
     unsigned count = 0;
-    const unsigned base = (PASS == 2 && i < A.ni) ? A.cnt[i] : 0;
-    for (uint64_t j0 = 0; j0 < A.nj; j0 += SK_TILE) {
-        const int n = (int)((A.nj - j0) < SK_TILE ? (A.nj - j0) : SK_TILE);
-        __syncthreads();
-        for (int t = threadIdx.x; t < 8 * SK_TILE; t += SK_THREADS) {
-            const int a = t / SK_TILE, jj = t % SK_TILE;
-            if (jj < n) tile[a][jj] = A.jp[a][j0 + jj];
-        }
-        __syncthreads();
-        for (int jj = 0; jj < n; ++jj) {
-            double jp[8];
-            for (int a = 0; a < 8; ++a) jp[a] = tile[a][jj];
-            double p0[6], pre[6], m, e2;
-            const bool kep = sk_kepler(ip, jp, dt, flag, p0, pre, &m, &e2);
-            if (PASS == 1) {
-                count += kep ? 1u : 0u;
-                continue;
-            }
-            if (kep) {
-                if (i < A.ni) {
-                    A.queue_j[base + count] = (unsigned)(j0 + jj);
-                    A.queue_i[base + count] = (unsigned)i;
-                }
-                ++count;
-                continue;
-            }
+    unsigned lanes = 0;             // this i's lanes of a warp
+    for (int k = 0; k < 32; k += 1 << li) lanes |= 1u << (k + ii);
+    int b = 0;
+    for (uint64_t j0 = 0; j0 < A.nj; j0 += J, b ^= 1) {
+        const uint64_t j = j0 + row < A.nj ? j0 + row : A.nj - 1;
+        double jp[8];
+#pragma unroll
+        for (int a = 0; a < 8; ++a) jp[a] = A.jp[a][j];
+        double p0[6], pre[6], m, e2;
+        sk_start(ip, jp, dt, flag, p0, pre, &m, &e2);
+        const bool far = takes_leapfrog(m, pre);
+        double t[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+        if (far) {
             double p1[6];
             two_body_leapfrog(dt, m, e2, pre, p1);
-            if (flag == 1) {
-                p1[0] -= p1[3] * dt;
-                p1[1] -= p1[4] * dt;
-                p1[2] -= p1[5] * dt;
+            if (flag == 1) pair_drift(p1, p1 + 3, dt, true);
+            pair_term(jp[0], m, p0, p1, t);
+        }
+#pragma unroll
+        for (int c = 0; c < NO; ++c) buf[b][c][tid] = t[c];
+        const unsigned v = __ballot_sync(0xffffffffu,
+                                         !far && j0 + row < A.nj);
+        if ((tid & 31) == 0) near[b][tid >> 5] = v;
+        __syncthreads();
+        if (sums) {
+            const int n = A.nj - j0 < (uint64_t)J ? (int)(A.nj - j0) : J;
+            const double *q = &buf[b][row][ii];
+#pragma unroll 8
+            for (int k = 0; k < n; ++k) o += q[k << li];
+        } else if (queues) {
+            unsigned f[T / 32], n = 0;
+#pragma unroll
+            for (int k = 0; k < T / 32; ++k) {
+                f[k] = near[b][k] & lanes;
+                n += __popc(f[k]);
             }
-            const double mu = jp[0] / m;
-            for (int q = 0; q < 6; ++q) o[q] += mu * (p1[q] - p0[q]);
+            if (n) {
+                unsigned long long at = atomicAdd(&A.rep->pairs,
+                                                  (unsigned long long)n);
+#pragma unroll
+                for (int k = 0; k < T / 32; ++k)
+                    for (; f[k]; f[k] &= f[k] - 1, ++at, ++count)
+                        if (at < A.cap) {
+                            const int l = 32 * k + __ffs((int)f[k]) - 1;
+                            A.queue_j[at] = (unsigned)(j0 + (l >> li));
+                            A.queue_i[at] = (unsigned)i;
+                            A.queue_r[at] = count;
+                        }
+            }
         }
     }
-    if (i >= A.ni) return;
-    if (PASS == 1) {
-        A.cnt[i] = count;
-    } else {
-        for (int q = 0; q < 6; ++q) A.out[q][i] = o[q];
-    }
+    if (sums && i0 + ii < A.ni) A.out[row][i] = o;
+    if (queues) A.cnt[i] = count;
 }
 
-// SPLIT mode of the two passes (flags -1 and +1): FP32 pair arithmetic on
+// The i's a block of the pass: as many (up to 16, the six sums and the
+// queue of each have to fit the block) as leave 600 blocks.
+int sk_li(uint64_t ni)
+{
+    int li = 4;
+    while (li > 0 && (ni >> li) < 600) --li;
+    return li;
+}
+
+// SPLIT mode of the pass (flags -1 and +1): FP32 pair arithmetic on
 // the packed double-single records.  In the leapfrog branch the pair's
 // change over the step has a closed form: with the midpoint position
 // b = r0 + flag v0 dt/2 and a = -m b / |b|^3 (softened), the velocity
@@ -304,12 +344,10 @@ k_sakura_pass(const SakuraArgs A)
 // sakura_kernel_common.h:45-91 with :151-164), so each pair is one
 // acceleration evaluation formed directly as increments (no difference of
 // nearly equal FP32 states).  The branch test is the reference's
-// (r^2 > (64 m / v^2)^2, sakura_kernel_common.h:109-123) in FP32; both
-// passes take the same decisions.  Kepler-branch pairs go to the same
+// (r^2 > (64 m / v^2)^2, sakura_kernel_common.h:109-123) in FP32.  Kepler-branch pairs go to the same
 // queue and fp64 solver as in EXACT mode.
 constexpr int SKS_TILE = 256;
 
-template <int PASS>
 __global__ void __launch_bounds__(SK_THREADS)
 k_sakura_split_pass(const SakuraArgs A, const float4 *irec, const float4 *jrec)
 {
@@ -323,7 +361,6 @@ k_sakura_split_pass(const SakuraArgs A, const float4 *irec, const float4 *jrec)
     float part[6] = {0, 0, 0, 0, 0, 0};
     int run = 0;
     unsigned count = 0;
-    const unsigned base = (PASS == 2 && i < A.ni) ? A.cnt[i] : 0;
     for (uint64_t j0 = 0; j0 < A.nj; j0 += SKS_TILE) {
         const int n = (int)((A.nj - j0) < SKS_TILE ? (A.nj - j0) : SKS_TILE);
         __syncthreads();
@@ -346,14 +383,18 @@ k_sakura_split_pass(const SakuraArgs A, const float4 *irec, const float4 *jrec)
             const float v2 = fmaf(uz, uz, fmaf(uy, uy, ux * ux));
             const float R = 64.0f * (m / v2);
             if (!(r2p > R * R)) {           // Kepler branch
-                if (PASS == 2 && i < A.ni) {
-                    A.queue_j[base + count] = (unsigned)(j0 + jj);
-                    A.queue_i[base + count] = (unsigned)i;
+                if (i < A.ni) {
+                    const unsigned long long at =
+                        atomicAdd(&A.rep->pairs, 1ull);
+                    if (at < A.cap) {
+                        A.queue_j[at] = (unsigned)(j0 + jj);
+                        A.queue_i[at] = (unsigned)i;
+                        A.queue_r[at] = count;
+                    }
                 }
                 ++count;
                 continue;
             }
-            if (PASS == 1) continue;
             const float bx = fmaf(ux, fl * hdt, dx), by = fmaf(uy, fl * hdt, dy),
                         bz = fmaf(uz, fl * hdt, dz);
             const float r2b = fmaf(bz, bz, fmaf(by, by, bx * bx));
@@ -377,15 +418,12 @@ k_sakura_split_pass(const SakuraArgs A, const float4 *irec, const float4 *jrec)
         }
     }
     if (i >= A.ni) return;
-    if (PASS == 1) {
-        A.cnt[i] = count;
-    } else {
-        for (int q = 0; q < 6; ++q) A.out[q][i] = o[q] + (double)part[q];
-    }
+    A.cnt[i] = count;
+    for (int q = 0; q < 6; ++q) A.out[q][i] = o[q] + (double)part[q];
 }
 
-// Exclusive scan of n counts in place (one block; returns the total).
-__global__ void k_scan(unsigned *x, uint64_t n, unsigned long long *total)
+// Exclusive scan of n counts in place (one block).
+__global__ void k_scan(unsigned *x, uint64_t n)
 {
     __shared__ unsigned long long carry;
     __shared__ unsigned long long part[1024];
@@ -408,26 +446,22 @@ __global__ void k_scan(unsigned *x, uint64_t n, unsigned long long *total)
         if (threadIdx.x == blockDim.x - 1) carry += part[threadIdx.x];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *total = carry;
 }
 
-// Step 4: one thread per queued pair.
-__global__ void __launch_bounds__(128)
-k_sakura_kepler(const SakuraArgs A, uint64_t nq, unsigned *err)
+// Step 3: one thread per queued pair; its contribution goes to its place in
+// (i, j) order.
+__device__ __forceinline__ void sk_solve(const SakuraArgs &A, uint64_t q,
+                                         const MlpSmem &S, unsigned *bins)
 {
-    __shared__ MlpSmem S;
-    if (A.use_mlp) mlp_stage(S, A.mlp);
-    __syncthreads();
-    const uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= nq) return;
     const uint64_t i = A.queue_i[q], j = A.queue_j[q];
+    const uint64_t at = (uint64_t)A.cnt[i] + A.queue_r[q];
     double ip[8], jp[8];
     for (int a = 0; a < 8; ++a) {
         ip[a] = A.ip[a][i];
         jp[a] = A.jp[a][j];
     }
     double p0[6], pre[6], m, e2, p1[6];
-    sk_kepler(ip, jp, A.dt, A.flag, p0, pre, &m, &e2);
+    sk_start(ip, jp, A.dt, A.flag, p0, pre, &m, &e2);
     KepCtx<double> ctx = {0, A.budget, 0, false, false, 0.0};
     ctx.form = A.form;
     if (A.use_mlp) {
@@ -447,23 +481,66 @@ k_sakura_kepler(const SakuraArgs A, uint64_t nq, unsigned *err)
         p1[2] -= p1[5] * A.dt;
     }
     const double mu = jp[0] / m;
-    for (int c = 0; c < 6; ++c) A.contrib[6 * q + c] = mu * (p1[c] - p0[c]);
-    if (A.iters) A.iters[q] = (int)ctx.iterations;
-    if (ctx.exhausted) atomicOr(err, (unsigned)DERR_KEPLER_BUDGET);
+    for (int c = 0; c < 6; ++c) A.contrib[6 * at + c] = mu * (p1[c] - p0[c]);
+    atomicAdd(&bins[ctx.iterations < 64 ? ctx.iterations : 64], 1u);
+    if (ctx.exhausted) atomicOr(&A.rep->err, (unsigned)DERR_KEPLER_BUDGET);
 }
 
-// Step 5: add each i's queued contributions in queue (= j) order.
-__global__ void k_sakura_gather(const SakuraArgs A, uint64_t nq)
+__global__ void __launch_bounds__(SK_THREADS)
+k_sakura_kepler(const SakuraArgs A)
 {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ MlpSmem S;
+    __shared__ unsigned bins[65];
+    const uint64_t nq = A.rep->pairs;
+    if (nq > A.cap) return;           // the host repeats the sweep
+    if (A.use_mlp) mlp_stage(S, A.mlp);
+    if (threadIdx.x < 65) bins[threadIdx.x] = 0;
+    __syncthreads();
+    for (uint64_t q = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nq;
+         q += (uint64_t)gridDim.x * blockDim.x)
+        sk_solve(A, q, S, bins);
+    __syncthreads();
+    if (threadIdx.x < 65 && bins[threadIdx.x])
+        atomicAdd(&A.rep->hist[threadIdx.x],
+                  (unsigned long long)bins[threadIdx.x]);
+}
+
+// Step 4: add each i's queued contributions in queue (= j) order.  A warp an
+// i: 32 contributions at a time come to shared memory coalesced, the next
+// 32 while six lanes add (one thread an i, 48-byte strides, the form this
+// replaces: 1.42 ms at N = 4096, where the heaviest body has thousands; now
+// 0.18 ms).
+__global__ void __launch_bounds__(SK_THREADS)
+k_sakura_gather(const SakuraArgs A)
+{
+    __shared__ double part[SK_THREADS / 32][6 * 32];
+    const uint64_t nq = A.rep->pairs;
+    if (nq > A.cap) return;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t i = (uint64_t)blockIdx.x * (SK_THREADS / 32) + w;
     if (i >= A.ni) return;
-    const uint64_t b = A.cnt[i];
-    const uint64_t e = (i + 1 < A.ni) ? A.cnt[i + 1] : nq;
-    double o[6];
-    for (int c = 0; c < 6; ++c) o[c] = A.out[c][i];
-    for (uint64_t q = b; q < e; ++q)
-        for (int c = 0; c < 6; ++c) o[c] += A.contrib[6 * q + c];
-    for (int c = 0; c < 6; ++c) A.out[c][i] = o[c];
+    const uint64_t b = 6 * (uint64_t)A.cnt[i];
+    const uint64_t e = 6 * ((i + 1 < A.ni) ? (uint64_t)A.cnt[i + 1] : nq);
+    double o = lane < 6 ? A.out[lane][i] : 0.0, x[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k)
+        x[k] = b + 32 * k + lane < e ? A.contrib[b + 32 * k + lane] : 0.0;
+    for (uint64_t q = b; q < e; q += 192) {
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 6; ++k) part[w][32 * k + lane] = x[k];
+        __syncwarp();
+        const uint64_t nx = q + 192 + lane;
+#pragma unroll
+        for (int k = 0; k < 6; ++k)
+            x[k] = nx + 32 * k < e ? A.contrib[nx + 32 * k] : 0.0;
+        if (lane < 6) {
+            const int n = e - q < 192 ? (int)(e - q) : 192;
+#pragma unroll 8
+            for (int k = lane; k < n; k += 6) o += part[w][k];
+        }
+    }
+    if (lane < 6) A.out[lane][i] = o;
 }
 
 }  // namespace tg
@@ -475,14 +552,14 @@ namespace {
 struct SakuraWork {
     unsigned *cnt = nullptr;
     size_t cnt_cap = 0;
-    unsigned *qi = nullptr, *qj = nullptr;
+    unsigned *qi = nullptr, *qj = nullptr, *qr = nullptr;
     double *contrib = nullptr;
-    int *iters = nullptr;
     size_t q_cap = 0;
-    unsigned long long *total = nullptr;
-    unsigned *err = nullptr;
+    SakuraReport *rep = nullptr;
+    unsigned *err = nullptr;          // kepler_pairs' error word
     float4 *rec = nullptr;            // SPLIT mode: packed i and j records
     size_t rec_cap = 0;
+    int sms = 0;
 };
 
 SakuraWork g_work;
@@ -490,18 +567,20 @@ MlpParams g_mlp;
 bool g_have_mlp = false;
 int g_kepler_form = KEP_REFERENCE;   // tupan_gb300_kepler_set_form
 
-int grow_queue(size_t nq)
+int grow_queue(size_t cap)
 {
-    if (nq <= g_work.q_cap) return 0;
+    if (cap <= g_work.q_cap) return 0;
     cudaFree(g_work.qi);
     cudaFree(g_work.qj);
+    cudaFree(g_work.qr);
     cudaFree(g_work.contrib);
-    cudaFree(g_work.iters);
-    size_t cap = nq + nq / 2 + 1024;
+    g_work.qi = g_work.qj = g_work.qr = nullptr;
+    g_work.contrib = nullptr;
+    g_work.q_cap = 0;
     if (cudaMalloc((void **)&g_work.qi, cap * sizeof(unsigned)) != cudaSuccess ||
         cudaMalloc((void **)&g_work.qj, cap * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc((void **)&g_work.contrib, cap * 6 * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void **)&g_work.iters, cap * sizeof(int)) != cudaSuccess)
+        cudaMalloc((void **)&g_work.qr, cap * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc((void **)&g_work.contrib, cap * 6 * sizeof(double)) != cudaSuccess)
         return 1;
     g_work.q_cap = cap;
     return 0;
@@ -618,13 +697,15 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
     if (use_mlp && !g_have_mlp) return ST_BAD_ARGUMENT;
     if (ni == 0) return ST_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    if (!g_work.err && (cudaMalloc((void **)&g_work.err, sizeof(unsigned)) !=
-                            cudaSuccess))
-        return ST_CUDA;
-    if (!g_work.total &&
-        cudaMalloc((void **)&g_work.total, sizeof(unsigned long long)) !=
-            cudaSuccess)
-        return ST_CUDA;
+    if (!g_work.rep) {
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess ||
+            cudaDeviceGetAttribute(&g_work.sms, cudaDevAttrMultiProcessorCount,
+                                   dev) != cudaSuccess ||
+            cudaMalloc((void **)&g_work.rep, sizeof(SakuraReport)) !=
+                cudaSuccess)
+            return ST_CUDA;
+    }
     if (ni > g_work.cnt_cap) {
         cudaFree(g_work.cnt);
         if (cudaMalloc((void **)&g_work.cnt, ni * sizeof(unsigned)) != cudaSuccess)
@@ -647,8 +728,10 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
     A.use_mlp = use_mlp;
     A.form = g_kepler_form;
     A.mlp = g_mlp;
-    cudaMemsetAsync(g_work.err, 0, sizeof(unsigned), st);
+    A.rep = g_work.rep;
     const unsigned blocks = (unsigned)((ni + SK_THREADS - 1) / SK_THREADS);
+    const int li = sk_li(ni);
+    const unsigned eblocks = (unsigned)((ni + (1u << li) - 1) >> li);
     const float4 *irec = nullptr, *jrec = nullptr;
     if (mode == MODE_SPLIT) {
         bool same = ni == nj;
@@ -671,51 +754,40 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
         irec = g_work.rec;
         jrec = same ? g_work.rec : g_work.rec + ni * 3;
     }
-    if (mode == MODE_SPLIT)
-        k_sakura_split_pass<1><<<blocks, SK_THREADS, 0, st>>>(A, irec, jrec);
-    else
-        k_sakura_pass<1><<<blocks, SK_THREADS, 0, st>>>(A);
-    k_scan<<<1, 1024, 0, st>>>(g_work.cnt, ni, g_work.total);
-    g_launch_count += 2;
-    unsigned long long nq = 0;
-    if (cudaMemcpyAsync(&nq, g_work.total, sizeof(nq), cudaMemcpyDeviceToHost,
-                        st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return ST_CUDA;
-    if (grow_queue(nq ? nq : 1)) return ST_CUDA;
-    A.queue_i = g_work.qi;
-    A.queue_j = g_work.qj;
-    A.contrib = g_work.contrib;
-    A.iters = kepler_iters ? g_work.iters : nullptr;
-    if (mode == MODE_SPLIT)
-        k_sakura_split_pass<2><<<blocks, SK_THREADS, 0, st>>>(A, irec, jrec);
-    else
-        k_sakura_pass<2><<<blocks, SK_THREADS, 0, st>>>(A);
-    g_launch_count += 1;
-    if (nq) {
-        k_sakura_kepler<<<(unsigned)((nq + 127) / 128), 128, 0, st>>>(
-            A, nq, g_work.err);
-        k_sakura_gather<<<(unsigned)((ni + 127) / 128), 128, 0, st>>>(A, nq);
-        g_launch_count += 2;
+    // room for a pair in 32 (Salpeter spheres: 1 in 16 at N = 256, 125 at
+    // 4096), at most 2^20 to begin with; the counts decide
+    unsigned long long want = ni * nj / 32 + 4096;
+    if (want > 1ull << 20) want = 1ull << 20;
+    SakuraReport r;
+    for (;;) {
+        if (grow_queue(want)) return ST_CUDA;
+        A.queue_i = g_work.qi;
+        A.queue_j = g_work.qj;
+        A.queue_r = g_work.qr;
+        A.cap = g_work.q_cap;
+        A.contrib = g_work.contrib;
+        cudaMemsetAsync(g_work.rep, 0, sizeof(SakuraReport), st);
+        if (mode == MODE_SPLIT)
+            k_sakura_split_pass<<<blocks, SK_THREADS, 0, st>>>(A, irec, jrec);
+        else
+            k_sakura_pass<<<eblocks, SK_THREADS, 0, st>>>(A, li);
+        k_scan<<<1, 1024, 0, st>>>(g_work.cnt, ni);
+        // the solves stride over the queue, whose length only the device
+        // knows: five blocks of 96 registers a thread fill an SM
+        k_sakura_kepler<<<(unsigned)(5 * g_work.sms), SK_THREADS, 0, st>>>(A);
+        k_sakura_gather<<<(unsigned)((ni + 3) / 4), SK_THREADS, 0, st>>>(A);
+        g_launch_count += 4;
+        if (cudaMemcpyAsync(&r, g_work.rep, sizeof(r), cudaMemcpyDeviceToHost,
+                            st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return ST_CUDA;
+        if (r.pairs <= A.cap) break;
+        want = r.pairs + r.pairs / 4;
     }
-    unsigned h = 0;
-    if (cudaMemcpyAsync(&h, g_work.err, sizeof(unsigned),
-                        cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return ST_CUDA;
-    if (n_kepler) *n_kepler = nq;
-    if (kepler_iters) {
-        for (int k = 0; k < 65; ++k) kepler_iters[k] = 0;
-        if (nq) {
-            int *hi = (int *)malloc(nq * sizeof(int));
-            if (!hi) return ST_CUDA;
-            cudaMemcpy(hi, g_work.iters, nq * sizeof(int), cudaMemcpyDeviceToHost);
-            for (unsigned long long q = 0; q < nq; ++q)
-                kepler_iters[hi[q] < 64 ? hi[q] : 64] += 1;
-            free(hi);
-        }
-    }
-    return h ? ST_DEVICE : ST_OK;
+    if (n_kepler) *n_kepler = r.pairs;
+    if (kepler_iters)
+        for (int k = 0; k < 65; ++k) kepler_iters[k] = (long long)r.hist[k];
+    return r.err ? ST_DEVICE : ST_OK;
 }
 
 // ===========================================================================

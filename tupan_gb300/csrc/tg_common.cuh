@@ -119,6 +119,10 @@ struct Sweep {
     // runs (ni is then its upper bound, used for the launch shape): a sweep
     // over a set whose size the GPU decides, launched without a host sync.
     const unsigned *ni_dev;
+    // Sakura: single-step solves a pair may take, and the device error word
+    // (launch_exact fills both in)
+    long long budget;
+    unsigned *err;
 };
 
 // Launch configuration of the FP32-split sweep, chosen by the autotuner.

@@ -621,39 +621,56 @@ __device__ void kep_solve(R dt, R m, R e2, const R *p0, R *p1, KepCtx<R> &c)
     for (int q = 0; q < 6; ++q) p1[q] = p[q];
 }
 
+// r += v h (or -=), a drift of the pair's relative state
+template <typename R>
+__device__ __forceinline__ void pair_drift(R *r, const R *v, R h, bool back)
+{
+    R x[3];
+    muls<3>(key_of(v[0], v[1], v[2], h), {v[0], v[1], v[2]}, {h, h, h}, x);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) r[c] = back ? r[c] - x[c] : r[c] + x[c];
+}
+
 // leapfrog + get_acc, sakura_kernel_common.h:24-91
 template <typename R>
-__device__ void two_body_leapfrog(R dt, R m, R e2, const R *p0, R *p1)
+__device__ __forceinline__ void two_body_leapfrog(R dt, R m, R e2,
+                                                  const R *p0, R *p1)
 {
-    R half = dt / R(2);
-    R rx = p0[0], ry = p0[1], rz = p0[2];
-    R vx = p0[3], vy = p0[4], vz = p0[5];
-    rx += vx * half;
-    ry += vy * half;
-    rz += vz * half;
-    R r2 = rx * rx + ry * ry + rz * rz;
-    R q = masked_inv_r2(r2, e2);
-    R k = q * sqrt(q);
-    R mk = m * k;
-    R ax = -mk * rx, ay = -mk * ry, az = -mk * rz;
-    vx += ax * dt;
-    vy += ay * dt;
-    vz += az * dt;
-    rx += vx * half;
-    ry += vy * half;
-    rz += vz * half;
-    p1[0] = rx; p1[1] = ry; p1[2] = rz;
-    p1[3] = vx; p1[4] = vy; p1[5] = vz;
+    const R half = dt / R(2);
+    R r[3] = {p0[0], p0[1], p0[2]}, v[3] = {p0[3], p0[4], p0[5]};
+    pair_drift(r, v, half, false);
+    const uint32_t kr = key_of(r[0], r[1], r[2]);
+    R p[3], q, w, k[1], a[3], x[3];
+    muls<3>(kr, r, r, p);
+    inv_root(p[0] + p[1] + p[2], e2, &q, &w);
+    muls<1>(key_of(q, w), {q}, {w}, k);
+    muls<1>(key_of(k[0], m), {m}, {k[0]}, k);
+    const R mk = -k[0];
+    muls<3>(soft::umax(kr, key_of(mk)), {mk, mk, mk}, r, a);
+    muls<3>(key_of(a[0], a[1], a[2], dt), a, {dt, dt, dt}, x);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) v[c] += x[c];
+    pair_drift(r, v, half, false);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        p1[c] = r[c];
+        p1[3 + c] = v[c];
+    }
 }
 
 // Branch test of twobody_solver, sakura_kernel_common.h:111-114
 template <typename R>
 __device__ __forceinline__ bool takes_leapfrog(R m, const R *p0)
 {
-    R r2 = p0[0] * p0[0] + p0[1] * p0[1] + p0[2] * p0[2];
-    R v2 = p0[3] * p0[3] + p0[4] * p0[4] + p0[5] * p0[5];
-    R Rr = R(64) * (m / v2);
-    return r2 > Rr * Rr;
+    R x[6], y[1];
+    muls<6>(key_of(p0[0], p0[1], p0[2], p0[3], p0[4], p0[5]),
+            {p0[0], p0[1], p0[2], p0[3], p0[4], p0[5]},
+            {p0[0], p0[1], p0[2], p0[3], p0[4], p0[5]}, x);
+    const R r2 = x[0] + x[1] + x[2];
+    const R v2 = x[3] + x[4] + x[5];
+    const R Rr = times64(quotient(m, v2));
+    muls<1>(key_of(Rr), {Rr}, {Rr}, y);
+    return greater(r2, y[0]);
 }
 
 template <typename R>
@@ -675,18 +692,14 @@ __device__ void evolve_pair(R dt, long long flag, R m, R e2, const R *p0,
     R p[6], q[6];
     for (int k = 0; k < 6; ++k) p[k] = p0[k];
     if (flag == -1) {
-        p[0] -= p[3] * dt;
-        p[1] -= p[4] * dt;
-        p[2] -= p[5] * dt;
+        pair_drift(p, p + 3, dt, true);
         two_body(dt, m, e2, p, q, c);
         for (int k = 0; k < 6; ++k) p[k] = q[k];
     }
     if (flag == 1) {
         two_body(dt, m, e2, p, q, c);
         for (int k = 0; k < 6; ++k) p[k] = q[k];
-        p[0] -= p[3] * dt;
-        p[1] -= p[4] * dt;
-        p[2] -= p[5] * dt;
+        pair_drift(p, p + 3, dt, true);
     }
     if (flag == -2) {
         p[0] -= p[3] * dt / R(2);
@@ -701,9 +714,7 @@ __device__ void evolve_pair(R dt, long long flag, R m, R e2, const R *p0,
     if (flag == 2) {
         two_body(dt / R(2), m, e2, p, q, c);
         for (int k = 0; k < 6; ++k) p[k] = q[k];
-        p[0] -= p[3] * dt;
-        p[1] -= p[4] * dt;
-        p[2] -= p[5] * dt;
+        pair_drift(p, p + 3, dt, true);
         two_body(dt / R(2), m, e2, p, q, c);
         for (int k = 0; k < 6; ++k) p[k] = q[k];
     }
@@ -723,6 +734,21 @@ __device__ __forceinline__ void pair_state(const R *ip, const R *jp, R *p0,
     p0[4] = ip[6] - jp[6];
     p0[5] = ip[7] - jp[7];
     *m = ip[0] + jp[0];
+}
+
+// (m_j / M)(p1 - p0), what a pair adds to its i's sums (sakura_kernel.c:52-57)
+template <typename R>
+__device__ __forceinline__ void pair_term(R jm, R m, const R *p0, const R *p1,
+                                          R *t)
+{
+    const R mu = quotient(jm, m);
+    R d[6], y[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) d[c] = p1[c] - p0[c];
+    muls<6>(key_of(mu, d[0], d[1], d[2], d[3], d[4], d[5]),
+            {mu, mu, mu, mu, mu, mu}, d, y);
+#pragma unroll
+    for (int c = 0; c < 6; ++c) t[c] = y[c];
 }
 
 // kepler_solver_kernel_common.h:39-79: particles a and b (m r e2 v) evolved

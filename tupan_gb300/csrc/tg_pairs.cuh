@@ -92,6 +92,16 @@ __device__ __forceinline__ double twice(double a)
                : 2.0 * a;
 }
 
+// 64 a, exact
+__device__ __forceinline__ float times64(float a) { return 64.0f * a; }
+
+__device__ __forceinline__ double times64(double a)
+{
+    return soft::range_key(a) < soft::RANGE
+               ? soft::make(soft::hi32(a) + (6u << 20), soft::lo32(a))
+               : 64.0 * a;
+}
+
 // r2 > 0 for an r2 that is not negative; fmax(a, o) for o not negative or
 // NaN (comparisons of doubles run on the FP64 pipe, those of their bits,
 // which order the same way, do not)
@@ -103,12 +113,20 @@ __device__ __forceinline__ bool positive(double r2)
     return b > 0 && b <= 0x7ff0000000000000ll;
 }
 
+// a > b for a, b not negative or NaN
+__device__ __forceinline__ bool greater(float a, float b) { return a > b; }
+
+__device__ __forceinline__ bool greater(double a, double b)
+{
+    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
+    return x > y && x <= 0x7ff0000000000000ll;
+}
+
 __device__ __forceinline__ float larger(float a, float o) { return fmax(a, o); }
 
 __device__ __forceinline__ double larger(double a, double o)
 {
-    const long long x = __double_as_longlong(a), y = __double_as_longlong(o);
-    return x > y && x <= 0x7ff0000000000000ll ? a : o;
+    return greater(a, o) ? a : o;
 }
 
 // e2_i + e2_j, kept while e2_j keeps its bits from one j to the next
