@@ -883,19 +883,29 @@ __global__ void __launch_bounds__(NT, MINB) ct_sweep(const CtLaunch L)
 // Sum the grid j-split partials in a fixed order and scatter to the
 // caller's order; nothing is written if a sweep CTA reported an error.
 template <int NO>
-__global__ void ct_finalize(const CtLaunch L, int gsplit)
+__global__ void __launch_bounds__(128)
+ct_finalize(const CtLaunch L, int gsplit)
 {
+    // one thread an (i, output), eight loads in flight before their
+    // additions
+    constexpr int RUN = 8;
     if (*(volatile unsigned *)L.err) return;
+    const int c = blockIdx.y;
     for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
          s < L.ni; s += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t o = L.perm[s];
+        const double *p = L.partial + (uint64_t)c * L.ni + s;
+        double a = p[0];
+        for (int y0 = 1; y0 < gsplit; y0 += RUN) {
+            double b[RUN];
 #pragma unroll
-        for (int c = 0; c < NO; ++c) {
-            double a = L.partial[(uint64_t)c * L.ni + s];
-            for (int y = 1; y < gsplit; ++y)
-                a += L.partial[((uint64_t)y * NO + c) * L.ni + s];
-            L.out[c][o] = a;
+            for (int k = 0; k < RUN; ++k)
+                b[k] = y0 + k < gsplit ? p[(uint64_t)(y0 + k) * NO * L.ni]
+                                       : 0.0;
+#pragma unroll
+            for (int k = 0; k < RUN; ++k)
+                if (y0 + k < gsplit) a += b[k];
         }
+        L.out[c][L.perm[s]] = a;
     }
 }
 
@@ -990,9 +1000,10 @@ static cudaError_t ct_run(const CtLaunch &L, int gsplit, cudaStream_t st)
     g_launch_count += 1;
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || gsplit == 1) return e;
-    uint64_t blocks = (L.ni + 255) / 256;
+    uint64_t blocks = (L.ni + 127) / 128;
     if (blocks > 152 * 8) blocks = 152 * 8;
-    ct_finalize<Op::NO><<<(unsigned)blocks, 256, 0, st>>>(L, gsplit);
+    ct_finalize<Op::NO><<<dim3((unsigned)blocks, Op::NO), 128, 0, st>>>(
+        L, gsplit);
     g_launch_count += 1;
     return cudaGetLastError();
 }

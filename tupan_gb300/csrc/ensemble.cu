@@ -417,9 +417,9 @@ __device__ __forceinline__ void batched_block(double *const *out, float eta,
             }
             const int q = u0 * NI + k;
             if (lane == 0 && u0 < units && q < ni) {
-                Op::finish(v, eta_d);
 #pragma unroll
-                for (int c = 0; c < NO; ++c) out[c][b + iv[k]] = v[c];
+                for (int c = 0; c < NO; ++c)
+                    out[c][b + iv[k]] = Op::finish(v[c], eta_d);
             }
         }
     }

@@ -388,9 +388,9 @@ __device__ void sub_split_sweep(SubState &S, int ilo, int ni, int jlo, int nj,
                 v[c] = c == Op::MAXC ? fmax(v[c], (double)part[c])
                                      : v[c] + (double)part[c];
         }
-        Op::finish(v, eta);
 #pragma unroll
-        for (int c = 0; c < Op::NO; ++c) S.f[first_out + c][ilo + t] = v[c];
+        for (int c = 0; c < Op::NO; ++c)
+            S.f[first_out + c][ilo + t] = Op::finish(v[c], eta);
     }
     __syncthreads();
 }

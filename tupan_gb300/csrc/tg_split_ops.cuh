@@ -3,7 +3,7 @@
 // single-CTA SIA recursion (sia.cu).  Each operator has NF float4 per
 // packed record, NO outputs, MAXC (index of a max-reduced output or -1),
 // a register image P of a record, pair() accumulating into float acc[NO]
-// and finish() in double on the reduced result.
+// and finish() in double on each reduced output.
 
 #pragma once
 
@@ -21,7 +21,7 @@ __device__ __forceinline__ void split2(double x, float &h, float &l)
 // Pair operators.  Each has:
 //   NF   float4 per record, NO outputs, MAXC index of a max-reduced output
 //   (or -1), I/J  register images of an i / j record, pair() accumulating
-//   into float acc[NO], finish() in double on the reduced result.
+//   into float acc[NO], finish() in double on each reduced output.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ float rsqrt_nr(float s)
 {
@@ -69,7 +69,7 @@ struct PhiSN {
         y = (s > h2) ? y : 0.0f;
         acc[0] = fmaf(-j.m, y, acc[0]);
     }
-    __device__ static void finish(double *, double) {}
+    __device__ static double finish(double v, double) { return v; }
 };
 using PhiS = PhiSN<true>;
 
@@ -92,7 +92,7 @@ struct AccSN {
         acc[1] = fmaf(mk, dy, acc[1]);
         acc[2] = fmaf(mk, dz, acc[2]);
     }
-    __device__ static void finish(double *, double) {}
+    __device__ static double finish(double v, double) { return v; }
 };
 using AccS = AccSN<true>;
 
@@ -126,7 +126,7 @@ struct AccJerkSN {
         acc[4] = fmaf(mk, fmaf(-al, dy, uy), acc[4]);
         acc[5] = fmaf(mk, fmaf(-al, dz, uz), acc[5]);
     }
-    __device__ static void finish(double *, double) {}
+    __device__ static double finish(double v, double) { return v; }
 };
 using AccJerkS = AccJerkSN<true>;
 
@@ -158,10 +158,9 @@ struct TstepSN {
         acc[0] += w2;
         acc[1] = fmaxf(w2, acc[1]);
     }
-    __device__ static void finish(double *v, double eta)
+    __device__ static double finish(double v, double eta)
     {
-        v[0] = eta / sqrt(1.0 + v[0]);
-        v[1] = eta / sqrt(1.0 + v[1]);
+        return eta / sqrt(1.0 + v);
     }
 };
 using TstepS = TstepSN<true>;
@@ -227,7 +226,7 @@ struct SnapSN {
         acc[4] = fmaf(mk, Jy, acc[4]);
         acc[5] = fmaf(mk, Jz, acc[5]);
     }
-    __device__ static void finish(double *, double) {}
+    __device__ static double finish(double v, double) { return v; }
 };
 using SnapS = SnapSN<true>;
 
