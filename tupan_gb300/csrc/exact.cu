@@ -10,6 +10,7 @@
 
 #include "tg_common.cuh"
 #include "tg_kepler.cuh"
+#include "tg_ordered.cuh"
 #include "tg_pairs.cuh"
 #include "tg_pn.cuh"
 
@@ -33,8 +34,8 @@ constexpr int EXACT_THREADS = 128;
 // blocks of 128 an SM) beat a prefetch at four blocks by 10 %: the chains of
 // dependent additions want warps.  Measured, double, Phi / AccJerk /
 // SnapCrackle / Tstep: N = 256 268 / 533 / 1216 / 687 us before, 17 / 19 /
-// 27 / 25 us now; N = 3001 2.98 / 6.09 / 14.1 / 7.70 ms, now 0.32 / 0.55 /
-// 1.41 / 0.65 ms; N = 32768 61 / 128 / 302 / 157 ms, now 21 / 51 / 141 /
+// 27 / 25 us now; N = 3001 2.98 / 6.09 / 14.1 / 7.70 ms, now 0.32 / 0.53 /
+// 1.40 / 0.65 ms; N = 32768 61 / 128 / 302 / 157 ms, now 21 / 51 / 141 /
 // 54 ms.  float takes four i a thread (one load of a j for four pairs, one
 // 16-byte store of a term): Phi + Acc at N = 10007 2.3 ms before, 0.62 ms.
 template <class Op, typename R, int T, int P, int BLK>
@@ -95,7 +96,7 @@ exact_terms(const Sweep s, const int li)
                 const int n = nj - j0 < (uint64_t)J ? (int)(nj - j0) : J;
                 const R *q = &buf[b][c][ii];
 #pragma unroll 8
-                for (int k = 0; k < n; ++k) o = Op::fold(c, o, q[k << li]);
+                for (int k = 0; k < n; ++k) o = fold<Op>(c, o, q[k << li]);
             }
         }
     }
@@ -105,6 +106,130 @@ exact_terms(const Sweep s, const int li)
         for (int a = 0; a < NA; ++a) ip[a] = ((const R *)s.ip[a])[i0 + ii];
         ((R *)s.out[c])[i0 + ii] = Op::finish(c, ip, o, s);
     }
+}
+
+// Few i against many j, double: one i a block, eight warps form the terms of
+// 256 j a tile while others sum the tile before.  A one-signed or max output
+// has a warp of its own (ordered_sum, or a maximum in any order); the others
+// share one, an output a lane, that adds term by term (their sums change
+// sign and binade too often for ordered_sum).  Bound: that chain of
+// additions, 64 cycles a term (AccJerk 100 x 8192 336 us, 273 of them the
+// chain), else the latency of a tile's pairs.  Measured against exact_terms
+// at one i a block: Phi 100 x 8192 387 -> 66 us, Tstep 576 -> 115, AccJerk
+// 447 -> 336, SnapCrackle 690 -> 405; NREG X at N = 256 33 -> 19 us.
+constexpr int FEW_T = 256;
+
+template <class Op>
+__host__ __device__ constexpr bool few_own(int c)
+{
+    return Op::one_signed(c) || Op::join(c) == JOIN_MAX;
+}
+
+template <class Op>
+__host__ __device__ constexpr int few_owned()
+{
+    int n = 0;
+    for (int c = 0; c < Op::NO; ++c) n += few_own<Op>(c) ? 1 : 0;
+    return n;
+}
+
+template <class Op>
+constexpr int few_threads()
+{
+    return FEW_T + 32 * (few_owned<Op>() + (few_owned<Op>() < Op::NO ? 1 : 0));
+}
+
+// The n-th output that has (own) or has not a warp of its own; NO if none.
+template <class Op>
+__device__ __forceinline__ int few_output(int n, bool own)
+{
+    int at = Op::NO;
+#pragma unroll
+    for (int c = Op::NO - 1; c >= 0; --c) {
+        int before = 0;
+        for (int q = 0; q < c; ++q) before += few_own<Op>(q) == own ? 1 : 0;
+        if (few_own<Op>(c) == own && before == n) at = c;
+    }
+    return at;
+}
+
+template <class Op>
+__global__ void __launch_bounds__(few_threads<Op>())
+exact_few(const Sweep s)
+{
+    constexpr int NA = Op::NA, NO = Op::NO;
+    constexpr int RUNS = FEW_T / ORD_RUN, SPAN = ORD_PITCH * ORD_K;
+    constexpr int ROW = RUNS * SPAN + 1;      // odd: outputs on other banks
+    __shared__ double buf[2][NO][ROW];
+    const uint64_t i = blockIdx.x, nj = s.nj;
+    if (s.ni_dev && i >= (uint64_t)*s.ni_dev) return;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const bool forms = tid < FEW_T;
+    const int w = (tid - FEW_T) >> 5;
+    const bool own = w < few_owned<Op>();
+    const int c = few_output<Op>(own ? w : lane, own);
+    double ip[NA], o = 0.0;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) ip[a] = ((const double *)s.ip[a])[i];
+    Softening<double> soft2;
+    if (nj) soft2.set(ip[4], ((const double *)s.jp[4])[0]);
+    // tile k is formed in step k and summed in step k + 1
+    const uint64_t tiles = (nj + FEW_T - 1) / FEW_T;
+    for (uint64_t k = 0; k <= tiles; ++k) {
+        if (forms) {
+            if (k < tiles) {
+                const uint64_t j = k * FEW_T + tid < nj ? k * FEW_T + tid
+                                                        : nj - 1;
+                double jp[NA], t[NO];
+#pragma unroll
+                for (int a = 0; a < NA; ++a)
+                    jp[a] = ((const double *)s.jp[a])[j];
+                Op::terms(ip, jp, t, s, soft2);
+#pragma unroll
+                for (int q = 0; q < NO; ++q)
+                    buf[k & 1][q][few_own<Op>(q)
+                                      ? tid / ORD_RUN * SPAN +
+                                            ord_at(tid % ORD_RUN)
+                                      : tid] =
+                        Op::join(q) == JOIN_SUB ? -t[q] : t[q];
+            }
+        } else if (k > 0 && c < NO) {
+            const uint64_t j0 = (k - 1) * FEW_T;
+            const int n = nj - j0 < (uint64_t)FEW_T ? (int)(nj - j0) : FEW_T;
+            const double *q = buf[(k - 1) & 1][c];
+            if (!own) {
+                // the next eight loads are under way while eight terms add
+                double x[8], y[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = e < n ? q[e] : -0.0;
+                for (int u = 0; u < n; u += 8) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        y[e] = u + 8 + e < n ? q[u + 8 + e] : -0.0;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) o = o + x[e];
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) x[e] = y[e];
+                }
+            } else if (Op::join(c) == JOIN_MAX) {
+                for (int u = lane; u < n; u += 32)
+                    o = larger(q[u / ORD_RUN * SPAN + ord_at(u % ORD_RUN)], o);
+            } else {
+                for (int r = 0; r * ORD_RUN < n; ++r)
+                    o = ordered_sum(o, q + r * SPAN,
+                                    n - r * ORD_RUN < ORD_RUN
+                                        ? n - r * ORD_RUN : ORD_RUN);
+            }
+        }
+        __syncthreads();
+    }
+    if (forms || c == NO) return;
+    if (own && Op::join(c) == JOIN_MAX) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1)
+            o = larger(__shfl_xor_sync(0xffffffffu, o, d), o);
+    }
+    if (!own || lane == 0) ((double *)s.out[c])[i] = Op::finish(c, ip, o, s);
 }
 
 // sakura_kernel.c:33-62: Sigma_j (m_j/M)(two-body step - initial state).
@@ -123,7 +248,8 @@ struct SakuraPair {
         if (c.exhausted) atomicOr(s.err, (unsigned)DERR_KEPLER_BUDGET);
         pair_term(jp[0], m, p0, p1, t);
     }
-    __device__ static R fold(int, R o, R t) { return o + t; }
+    __device__ static constexpr int join(int) { return JOIN_ADD; }
+    __device__ static constexpr bool one_signed(int) { return false; }
     __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
 };
 
@@ -156,6 +282,20 @@ static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
     constexpr int T = EXACT_THREADS;
     constexpr int P = sizeof(R) == 8 ? 1 : Op::WIDE ? 1 : 4;
     constexpr int BLK = sizeof(R) == 8 ? (Op::WIDE ? 4 : 8) : 6;
+    if constexpr (sizeof(R) == 8) {
+        // One i a block where its sums are the bound: sums with warps of
+        // their own (Phi, Tstep) win up to 5000 i (Phi at 3001 x 3001 267 us
+        // against 320, at 8192 equal; Tstep at 5000 x 5000 1.61 against 1.81
+        // ms, at 8192 7 % slower), sums that share one while no SM has more
+        // than two blocks (AccJerk 300 x 8192 380 us against 477, 600 x 3000
+        // equal, 1000 x 1000 137 against 107).
+        constexpr uint64_t most = few_owned<Op>() == Op::NO ? 5000 : 2 * 152;
+        if (s.ni <= most) {
+            exact_few<Op><<<(unsigned)s.ni, few_threads<Op>(), 0, st>>>(s);
+            g_launch_count += 1;
+            return cudaGetLastError();
+        }
+    }
     // As many i a block as leave 600 blocks (four an SM): more i share a j
     // load and fill the warps that add, fewer leave SMs idle (AccJerk at
     // N = 3001: 751 blocks of 4 i 0.55 ms, 376 of 8 i 0.70 ms; at 32768

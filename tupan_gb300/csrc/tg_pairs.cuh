@@ -185,10 +185,21 @@ __device__ __forceinline__ void inv_root(double r2, double h2, double *q,
 }
 
 // Each operator gives the terms one j adds to the sums of one i (terms),
-// how a term joins its sum (fold; sums start from zero) and the last step
-// of each output (finish).  Terms of different j are independent, so they
+// how a term joins its sum (join: added, subtracted or the larger kept; sums
+// start from zero; fold does it), whether an output's terms nearly all have
+// one sign (one_signed: ordered_sum's fast case) and the last step of each
+// output (finish).  Terms of different j are independent, so they
 // may be formed in any order; folding them in j order keeps the
 // reference's bits.
+enum Join : int { JOIN_ADD = 0, JOIN_SUB = 1, JOIN_MAX = 2 };
+
+template <class Op, typename R>
+__device__ __forceinline__ R fold(int c, R o, R t)
+{
+    const int j = Op::join(c);
+    return j == JOIN_MAX ? larger(t, o) : j == JOIN_SUB ? o - t : o + t;
+}
+
 template <class Op, typename R>
 __device__ __forceinline__ void fold_pair(const R *ip, const R *jp, R *o,
                                           const Sweep &s,
@@ -197,7 +208,7 @@ __device__ __forceinline__ void fold_pair(const R *ip, const R *jp, R *o,
     R t[Op::NO];
     Op::terms(ip, jp, t, s, soft2);
 #pragma unroll
-    for (int c = 0; c < Op::NO; ++c) o[c] = Op::fold(c, o[c], t[c]);
+    for (int c = 0; c < Op::NO; ++c) o[c] = fold<Op>(c, o[c], t[c]);
 }
 
 // phi_kernel_common.h:7-32
@@ -219,7 +230,8 @@ struct PhiPair {
         muls<1>(key_of(a[0], w), a, b, x);
         t[0] = x[0];
     }
-    __device__ static R fold(int, R o, R t) { return o - t; }
+    __device__ static constexpr int join(int) { return JOIN_SUB; }
+    __device__ static constexpr bool one_signed(int) { return true; }
     __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
 };
 
@@ -248,7 +260,8 @@ struct AccPair {
         t[1] = x[1];
         t[2] = x[2];
     }
-    __device__ static R fold(int, R o, R t) { return o - t; }
+    __device__ static constexpr int join(int) { return JOIN_SUB; }
+    __device__ static constexpr bool one_signed(int) { return false; }
     __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
 };
 
@@ -289,7 +302,8 @@ struct AccJerkPair {
 #pragma unroll
         for (int c = 0; c < 6; ++c) t[c] = y[c];
     }
-    __device__ static R fold(int, R o, R t) { return o - t; }
+    __device__ static constexpr int join(int) { return JOIN_SUB; }
+    __device__ static constexpr bool one_signed(int) { return false; }
     __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
 };
 
@@ -385,7 +399,8 @@ struct SnapCracklePair {
 #pragma unroll
         for (int n = 0; n < 6; ++n) t[n] = y[n];
     }
-    __device__ static R fold(int, R o, R t) { return o - t; }
+    __device__ static constexpr int join(int) { return JOIN_SUB; }
+    __device__ static constexpr bool one_signed(int) { return false; }
     __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
 };
 
@@ -429,10 +444,11 @@ struct TstepPair {
         t[0] = w2;
         t[1] = w2;
     }
-    __device__ static R fold(int c, R o, R t)
+    __device__ static constexpr int join(int c)
     {
-        return c == 0 ? o + t : larger(t, o);
+        return c == 0 ? JOIN_ADD : JOIN_MAX;
     }
+    __device__ static constexpr bool one_signed(int c) { return c == 0; }
     __device__ static R finish(int, const R *, R o, const Sweep &s)
     {
         R eta = R(s.scal[0]);
@@ -471,10 +487,11 @@ struct NregXPair {
 #pragma unroll
         for (int n = 0; n < 7; ++n) t[n] = y[n];
     }
-    __device__ static R fold(int c, R o, R t)
+    __device__ static constexpr int join(int c)
     {
-        return c < 3 || c == 6 ? o + t : o - t;
+        return c < 3 || c == 6 ? JOIN_ADD : JOIN_SUB;
     }
+    __device__ static constexpr bool one_signed(int c) { return c == 6; }
     __device__ static R finish(int c, const R *ip, R o, const Sweep &)
     {
         return c == 6 ? ip[0] * o : o;
@@ -507,7 +524,8 @@ struct NregVPair {
 #pragma unroll
         for (int n = 0; n < 4; ++n) t[n] = y[n];
     }
-    __device__ static R fold(int, R o, R t) { return o + t; }
+    __device__ static constexpr int join(int) { return JOIN_ADD; }
+    __device__ static constexpr bool one_signed(int c) { return c == 3; }
     __device__ static R finish(int c, const R *ip, R o, const Sweep &)
     {
         return c == 3 ? ip[0] * o : o;

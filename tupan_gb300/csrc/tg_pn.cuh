@@ -298,7 +298,8 @@ struct PnAccPair {
         t[1] = pa * dy + pb * uy;
         t[2] = pa * dz + pb * uz;
     }
-    __device__ static R fold(int, R o, R t) { return o + t; }
+    __device__ static constexpr int join(int) { return JOIN_ADD; }
+    __device__ static constexpr bool one_signed(int) { return false; }
     __device__ static R finish(int, const R *, R o, const Sweep &) { return o; }
 };
 
