@@ -89,6 +89,13 @@ class AbstractExtension(object):
         sig = abi.SIGNATURES[self.kernel_name]
         self.argtypes = tuple(kinds[k] for (k, _) in sig if k != "out")
         self.restypes = tuple(kinds[k] for (k, _) in sig if k == "out")
+        # where each input comes from: a count, an attribute of the i or j
+        # set, or a scalar
+        self._sources = tuple(
+            ("n" if arg in ("ni", "nj") else "a" if kind == "in" else "s",
+             arg[0] == "i", _ATTR.get(arg[1:], arg[1:]) if kind == "in"
+             else arg)
+            for (kind, arg) in sig if kind != "out")
 
     def _scalars(self, args):
         return dict(zip(self.scalar_names, args))
@@ -102,14 +109,11 @@ class AbstractExtension(object):
                 ips.register_auxiliary_attribute(attr, "real")
         scal = self._scalars(args)
         inargs = []
-        for kind, arg in abi.SIGNATURES[name]:
-            if kind == "out":
-                continue
-            if arg in ("ni", "nj"):
+        for kind, of_i, arg in self._sources:
+            if kind == "a":
+                inargs.append(getattr(ips if of_i else jps, arg))
+            elif kind == "n":
                 inargs.append(ips.n if arg == "ni" else jps.n)
-            elif kind == "in":
-                side = ips if arg[0] == "i" else jps
-                inargs.append(getattr(side, _ATTR.get(arg[1:], arg[1:])))
             else:
                 inargs.append(scal[arg])
         self._inargs = tuple(inargs)
