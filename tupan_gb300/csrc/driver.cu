@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "tg_common.cuh"
+#include "tg_pairs.cuh"
 
 #define TG_EXPORT extern "C" __attribute__((visibility("default")))
 
@@ -51,7 +52,7 @@ struct StepCtl {
     double tau;        // step of the current iteration
     unsigned long long min_ts_bits;   // min |dt_a| as ordered bits
     int done;          // 1 once |t| >= t_end: further steps are no-ops
-    int pad;
+    unsigned arrived;  // blocks of k_min_tstep that are through
     long long nsteps;
 };
 
@@ -80,21 +81,44 @@ __device__ __forceinline__ double d_block_tstep(double min_ts, double t,
     return min_bts;
 }
 
-__global__ void k_begin_step(StepCtl *c)
+struct Arrays {
+    double *m, *e2;
+    double *r[3], *v[3];        // current state (ps / ps1)
+    double *r0[3], *v0[3];      // copy at the start of the step (ps0)
+    double *f0[12], *f1[12];    // a(3) j(3) s(3) c(3) of ps0 and ps1
+    double *dt[2];              // tstep outputs (tstep, tstepij)
+};
+
+// The per-particle stages of a step.  Blocks of 64 threads, one component a
+// thread (blockIdx.y), so that 256 bodies spread over twelve SMs: the stages
+// are a few dependent FP64 operations and divisions, and blocks of 256 put
+// all of them on one SM's FP64 pipe (predict 7 us, correct 9.4 us there at
+// N = 256, now 3.7 and 4.2).  Divisions by 3, 5, 6, 12, .. take the integer
+// pipe (quotient: the same bits).
+constexpr int STAGE_T = 64;
+
+// Opens a step (one thread) and copies the state; every block decides by
+// itself whether the end time is reached.
+__global__ void k_begin_step(Arrays A, uint64_t n, StepCtl *c)
 {
-    if (threadIdx.x || blockIdx.x) return;
-    if (fabs(c->t) >= c->t_end) {
-        c->done = 1;
-        c->tau = 0.0;
-        return;
+    const bool done = fabs(c->t) >= c->t_end;
+    const int d = blockIdx.y;
+    if (threadIdx.x == 0 && blockIdx.x == 0 && d == 0) {
+        c->done = done ? 1 : 0;
+        c->tau = done ? 0.0 : d_base_tstep(c->t, c->t_end, c->eta);
+        if (!done) c->min_ts_bits = 0x7ff0000000000000ull;   // +inf
     }
-    c->done = 0;
-    c->tau = d_base_tstep(c->t, c->t_end, c->eta);
-    c->min_ts_bits = 0x7ff0000000000000ull;   // +inf
+    if (done) return;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        A.r0[d][i] = A.r[d][i];
+        A.v0[d][i] = A.v[d][i];
+    }
 }
 
-// min |dt_a| over particles; non-negative doubles order like their bits.
-__global__ void k_min_abs(const double *x, uint64_t n, StepCtl *c)
+// min |dt_a| over particles (non-negative doubles order like their bits);
+// the last block through turns it into the step.
+__global__ void k_min_tstep(const double *x, uint64_t n, StepCtl *c)
 {
     if (c->done) return;
     unsigned long long best = 0x7ff0000000000000ull;
@@ -107,41 +131,18 @@ __global__ void k_min_abs(const double *x, uint64_t n, StepCtl *c)
         unsigned long long o = __shfl_xor_sync(0xffffffffu, best, off);
         best = o < best ? o : best;
     }
-    if ((threadIdx.x & 31) == 0) atomicMin(&c->min_ts_bits, best);
-}
-
-__global__ void k_block_tstep(StepCtl *c)
-{
-    if (threadIdx.x || blockIdx.x || c->done) return;
-    double min_ts = __longlong_as_double((long long)c->min_ts_bits);
-    c->tau = d_block_tstep(min_ts, c->t, c->tau);
-}
-
-__global__ void k_end_step(StepCtl *c, double *tau_log, long long cap)
-{
-    if (threadIdx.x || blockIdx.x || c->done) return;
-    if (tau_log && c->nsteps < cap) tau_log[c->nsteps] = c->tau;
-    c->t += c->tau;
-    c->nsteps += 1;
-}
-
-struct Arrays {
-    double *m, *e2;
-    double *r[3], *v[3];        // current state (ps / ps1)
-    double *r0[3], *v0[3];      // copy at the start of the step (ps0)
-    double *f0[12], *f1[12];    // a(3) j(3) s(3) c(3) of ps0 and ps1
-    double *dt[2];              // tstep outputs (tstep, tstepij)
-};
-
-__global__ void k_copy_state(Arrays A, uint64_t n, const StepCtl *c)
-{
-    if (c->done) return;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        for (int d = 0; d < 3; ++d) {
-            A.r0[d][i] = A.r[d][i];
-            A.v0[d][i] = A.v[d][i];
-        }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMin(&c->min_ts_bits, best);
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    if (atomicAdd(&c->arrived, 1u) + 1u < gridDim.x) return;
+    c->arrived = 0;
+    __threadfence();
+    const unsigned long long m = atomicMin(&c->min_ts_bits,
+                                           0x7ff0000000000000ull);
+    c->tau = d_block_tstep(__longlong_as_double((long long)m), c->t, c->tau);
 }
 
 // Hn.epredict position/velocity updates (hermite.py:33-38, :83-88,
@@ -151,76 +152,87 @@ __global__ void k_predict(Arrays A, uint64_t n, const StepCtl *c)
 {
     if (c->done) return;
     const double tau = c->tau;
+    const int d = blockIdx.y;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        for (int d = 0; d < 3; ++d) {
-            const double a = A.f0[d][i];
-            const double v = A.v[d][i];
-            double rr, vv;
-            if (ORDER == 2) {
-                rr = (a * tau / 2 + v) * tau;
-                vv = a * tau;
-            } else if (ORDER == 4) {
-                const double j = A.f0[3 + d][i];
-                rr = ((j * tau / 3 + a) * tau / 2 + v) * tau;
-                vv = (j * tau / 2 + a) * tau;
-            } else if (ORDER == 6) {
-                const double j = A.f0[3 + d][i], s = A.f0[6 + d][i];
-                rr = (((s * tau / 4 + j) * tau / 3 + a) * tau / 2 + v) * tau;
-                vv = ((s * tau / 3 + j) * tau / 2 + a) * tau;
-            } else {
-                const double j = A.f0[3 + d][i], s = A.f0[6 + d][i],
-                             cr = A.f0[9 + d][i];
-                rr = ((((cr * tau / 5 + s) * tau / 4 + j) * tau / 3 + a) *
-                          tau / 2 + v) * tau;
-                vv = (((cr * tau / 4 + s) * tau / 3 + j) * tau / 2 + a) * tau;
-            }
-            A.r[d][i] = A.r[d][i] + rr;
-            A.v[d][i] = v + vv;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const double a = A.f0[d][i];
+        const double v = A.v[d][i];
+        double rr, vv;
+        if (ORDER == 2) {
+            rr = (a * tau / 2 + v) * tau;
+            vv = a * tau;
+        } else if (ORDER == 4) {
+            const double j = A.f0[3 + d][i];
+            rr = ((quotient(j * tau, 3.0) + a) * tau / 2 + v) * tau;
+            vv = (j * tau / 2 + a) * tau;
+        } else if (ORDER == 6) {
+            const double j = A.f0[3 + d][i], s = A.f0[6 + d][i];
+            rr = ((quotient((s * tau / 4 + j) * tau, 3.0) + a) * tau / 2 + v) *
+                 tau;
+            vv = ((quotient(s * tau, 3.0) + j) * tau / 2 + a) * tau;
+        } else {
+            const double j = A.f0[3 + d][i], s = A.f0[6 + d][i],
+                         cr = A.f0[9 + d][i];
+            rr = ((quotient(((quotient(cr * tau, 5.0) + s) * tau / 4 + j) * tau,
+                            3.0) + a) * tau / 2 + v) * tau;
+            vv = ((quotient((cr * tau / 4 + s) * tau, 3.0) + j) * tau / 2 + a) *
+                 tau;
         }
+        A.r[d][i] = A.r[d][i] + rr;
+        A.v[d][i] = v + vv;
+    }
 }
 
 // Hn.ecorrect (hermite.py:46-57, :96-119, :162-195, :238-283): velocities
-// first, positions from the corrected velocities.
+// first, positions from the corrected velocities.  `last`: the pass that
+// closes the step (no block reads the time or the count).
 template <int ORDER>
-__global__ void k_correct(Arrays A, uint64_t n, const StepCtl *c)
+__global__ void k_correct(Arrays A, uint64_t n, StepCtl *c, bool last,
+                          double *tau_log, long long cap)
 {
     if (c->done) return;
     const double tau = c->tau;
+    const int d = blockIdx.y;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        for (int d = 0; d < 3; ++d) {
-            const double a0 = A.f0[d][i], a1 = A.f1[d][i];
-            const double v0 = A.v0[d][i], r0 = A.r0[d][i];
-            double v1, r1;
-            if (ORDER == 2) {
-                v1 = ((a0 + a1) * tau / 2 + v0);
-                r1 = ((v0 + v1) * tau / 2 + r0);
-            } else if (ORDER == 4) {
-                const double j0 = A.f0[3 + d][i], j1 = A.f1[3 + d][i];
-                v1 = (((j0 - j1) * tau / 6 + (a0 + a1)) * tau / 2 + v0);
-                r1 = (((a0 - a1) * tau / 6 + (v0 + v1)) * tau / 2 + r0);
-            } else if (ORDER == 6) {
-                const double j0 = A.f0[3 + d][i], j1 = A.f1[3 + d][i];
-                const double s0 = A.f0[6 + d][i], s1 = A.f1[6 + d][i];
-                v1 = ((((s0 + s1) * tau / 12 + (j0 - j1)) * tau / 5 +
-                       (a0 + a1)) * tau / 2 + v0);
-                r1 = ((((j0 + j1) * tau / 12 + (a0 - a1)) * tau / 5 +
-                       (v0 + v1)) * tau / 2 + r0);
-            } else {
-                const double j0 = A.f0[3 + d][i], j1 = A.f1[3 + d][i];
-                const double s0 = A.f0[6 + d][i], s1 = A.f1[6 + d][i];
-                const double c0 = A.f0[9 + d][i], c1 = A.f1[9 + d][i];
-                v1 = (((((c0 - c1) * tau / 20 + (s0 + s1)) * tau / 3 +
-                        3 * (j0 - j1)) * tau / 14 + (a0 + a1)) * tau / 2 +
-                      v0);
-                r1 = (((((s0 - s1) * tau / 20 + (j0 + j1)) * tau / 3 +
-                        3 * (a0 - a1)) * tau / 14 + (v0 + v1)) * tau / 2 +
-                      r0);
-            }
-            A.v[d][i] = v1;
-            A.r[d][i] = r1;
+         i += (uint64_t)gridDim.x * blockDim.x) {
+        const double a0 = A.f0[d][i], a1 = A.f1[d][i];
+        const double v0 = A.v0[d][i], r0 = A.r0[d][i];
+        double v1, r1;
+        if (ORDER == 2) {
+            v1 = ((a0 + a1) * tau / 2 + v0);
+            r1 = ((v0 + v1) * tau / 2 + r0);
+        } else if (ORDER == 4) {
+            const double j0 = A.f0[3 + d][i], j1 = A.f1[3 + d][i];
+            v1 = ((quotient((j0 - j1) * tau, 6.0) + (a0 + a1)) * tau / 2 + v0);
+            r1 = ((quotient((a0 - a1) * tau, 6.0) + (v0 + v1)) * tau / 2 + r0);
+        } else if (ORDER == 6) {
+            const double j0 = A.f0[3 + d][i], j1 = A.f1[3 + d][i];
+            const double s0 = A.f0[6 + d][i], s1 = A.f1[6 + d][i];
+            v1 = ((quotient((quotient((s0 + s1) * tau, 12.0) + (j0 - j1)) * tau,
+                            5.0) + (a0 + a1)) * tau / 2 + v0);
+            r1 = ((quotient((quotient((j0 + j1) * tau, 12.0) + (a0 - a1)) * tau,
+                            5.0) + (v0 + v1)) * tau / 2 + r0);
+        } else {
+            const double j0 = A.f0[3 + d][i], j1 = A.f1[3 + d][i];
+            const double s0 = A.f0[6 + d][i], s1 = A.f1[6 + d][i];
+            const double c0 = A.f0[9 + d][i], c1 = A.f1[9 + d][i];
+            v1 = ((quotient((quotient((quotient((c0 - c1) * tau, 20.0) +
+                                       (s0 + s1)) * tau, 3.0) +
+                             3 * (j0 - j1)) * tau, 14.0) +
+                   (a0 + a1)) * tau / 2 + v0);
+            r1 = ((quotient((quotient((quotient((s0 - s1) * tau, 20.0) +
+                                       (j0 + j1)) * tau, 3.0) +
+                             3 * (a0 - a1)) * tau, 14.0) +
+                   (v0 + v1)) * tau / 2 + r0);
         }
+        A.v[d][i] = v1;
+        A.r[d][i] = r1;
+    }
+    if (last && threadIdx.x == 0 && blockIdx.x == 0 && d == 0) {
+        if (tau_log && c->nsteps < cap) tau_log[c->nsteps] = tau;
+        c->t += tau;
+        c->nsteps += 1;
+    }
 }
 
 // Kinetic energy 0.5 sum m v^2 and potential 0.5 sum m phi, fp64; block
@@ -290,10 +302,11 @@ int grow(void **p, size_t *have, size_t need)
     return 0;
 }
 
+// Blocks of STAGE_T threads for n particles, at most 32 an SM.
 unsigned grid_for(uint64_t n, int sms)
 {
-    uint64_t b = (n + 255) / 256;
-    uint64_t cap = (uint64_t)sms * 8;
+    uint64_t b = (n + STAGE_T - 1) / STAGE_T;
+    uint64_t cap = (uint64_t)sms * 32;
     return (unsigned)(b < 1 ? 1 : (b > cap ? cap : b));
 }
 
@@ -348,28 +361,27 @@ cudaError_t forces(Hermite *h, double *const *rr, double *const *vv,
 template <int ORDER>
 cudaError_t step_order(Hermite *h)
 {
-    const unsigned g = grid_for(h->n, h->sms);
+    const unsigned b = grid_for(h->n, h->sms);
+    const dim3 g(b, 3);
     cudaStream_t st = h->stream;
-    k_begin_step<<<1, 32, 0, st>>>(h->ctl);
+    k_begin_step<<<g, STAGE_T, 0, st>>>(h->A, h->n, h->ctl);
     if (h->adaptive) {
         const double *at[8] = {h->A.m, h->A.r[0], h->A.r[1], h->A.r[2],
                                h->A.e2, h->A.v[0], h->A.v[1], h->A.v[2]};
         cudaError_t e = sweep(h, K_TSTEP, at, h->A.dt, h->eta);
         if (e != cudaSuccess) return e;
-        k_min_abs<<<g, 256, 0, st>>>(h->A.dt[0], h->n, h->ctl);
-        k_block_tstep<<<1, 32, 0, st>>>(h->ctl);
+        k_min_tstep<<<b, STAGE_T, 0, st>>>(h->A.dt[0], h->n, h->ctl);
     }
-    k_copy_state<<<g, 256, 0, st>>>(h->A, h->n, h->ctl);
     cudaError_t e = forces(h, h->A.r0, h->A.v0, h->A.f0);
     if (e != cudaSuccess) return e;
-    k_predict<ORDER><<<g, 256, 0, st>>>(h->A, h->n, h->ctl);
+    k_predict<ORDER><<<g, STAGE_T, 0, st>>>(h->A, h->n, h->ctl);
     for (int pass = 0; pass < 2; ++pass) {
         e = forces(h, h->A.r, h->A.v, h->A.f1);
         if (e != cudaSuccess) return e;
-        k_correct<ORDER><<<g, 256, 0, st>>>(h->A, h->n, h->ctl);
+        k_correct<ORDER><<<g, STAGE_T, 0, st>>>(h->A, h->n, h->ctl, pass == 1,
+                                                h->tau_log, h->tau_cap);
     }
-    k_end_step<<<1, 32, 0, st>>>(h->ctl, h->tau_log, h->tau_cap);
-    g_launch_count += h->adaptive ? 8 : 6;
+    g_launch_count += h->adaptive ? 5 : 4;
     return cudaGetLastError();
 }
 
