@@ -328,13 +328,16 @@ split_sweep(const SplitLaunch L)
                             for (int q = 0; q < NP; ++q) pairfn(q, jp, p2[q]);
                         }
                     } else {
+                        // Paired: the whole tail is one run
+                        const int most = IsPaired<Op>::value ? TJ : FOLD;
 #pragma unroll 1
-                        for (int u = 0; u < FOLD && r0 + u * JS < n; ++u) {
+                        for (int u = 0; u < most && r0 + u * JS < n; ++u) {
                             const typename Op::P jp =
                                 Op::load(tile + (r0 + u * JS) * NF);
 #pragma unroll
                             for (int q = 0; q < NP; ++q) pairfn(q, jp, p2[q]);
                         }
+                        if (IsPaired<Op>::value) r0 = n;
                     }
                     // the run folds into the packed Kahan pairs of both i
 #pragma unroll
@@ -576,6 +579,10 @@ bool split_supported(int kernel)
            kernel == K_TSTEP || kernel == K_SNAP_CRACKLE || kernel == K_PNACC;
 }
 
+// Paired<Op> reduces like Op.
+template <class Op> struct FinalOp { using type = Op; };
+template <class Op> struct FinalOp<Paired<Op>> { using type = Op; };
+
 template <class Op, int NI, int JS, int NT, int MINB, bool X2 = false>
 static cudaError_t run_variant(const SplitLaunch &L, int gsplit,
                                cudaStream_t st)
@@ -589,7 +596,7 @@ static cudaError_t run_variant(const SplitLaunch &L, int gsplit,
     if (e != cudaSuccess || gsplit == 1) return e;
     uint64_t blocks = (L.ni + FINALIZE_I - 1) / FINALIZE_I;
     if (blocks > 152 * 8) blocks = 152 * 8;
-    split_finalize<Op><<<dim3((unsigned)blocks, Op::NO),
+    split_finalize<typename FinalOp<Op>::type><<<dim3((unsigned)blocks, Op::NO),
                          dim3(FINALIZE_I, FINALIZE_W), 0, st>>>(L, gsplit);
     g_launch_count += 1;
     return cudaGetLastError();
@@ -603,8 +610,26 @@ static cudaError_t run_op(const SplitLaunch &L, int variant, int gsplit,
     case 0: return run_variant<Op, 2, 1, 256, 2>(L, gsplit, st);
     case 1: return run_variant<Op, 1, 1, 256, 2>(L, gsplit, st);
     case 2: return run_variant<Op, 1, 4, 256, 2>(L, gsplit, st);
-    case 3: return run_variant<Op, 1, 16, 256, 2>(L, gsplit, st);
-    case 4: return run_variant<Op, 1, 32, 128, 4>(L, gsplit, st);
+    case 3:
+    case 4:
+        // The same sums with two i a thread in packed FP32 (Paired: equal
+        // bits), once that leaves blocks for every SM and, on 32 lanes, four
+        // tiles a block: 16 i a block on 16 lanes, 8 on 32.  1021 x 65536
+        // SnapCrackle on 32 lanes 272 -> 233 us, AccJerk on 16 165 -> 143,
+        // 3001 x 3001 SnapCrackle 74 -> 53; 64 x 65536, with a quarter of
+        // the blocks, would take 50 us against 37.
+        if constexpr (!std::is_void<typename X2Of<Op>::type>::value) {
+            const uint64_t ctas = (L.ni + (variant == 3 ? 15 : 7)) /
+                                  (variant == 3 ? 16 : 8) * gsplit;
+            if (variant == 3 && ctas >= 200)
+                return run_variant<Paired<Op>, 2, 16, 128, 4, true>(L, gsplit,
+                                                                    st);
+            if (variant == 4 && ctas >= 250 && L.jchunk >= 4 * SPLIT_TILE)
+                return run_variant<Paired<Op>, 2, 32, 128, 4, true>(L, gsplit,
+                                                                    st);
+        }
+        if (variant == 3) return run_variant<Op, 1, 16, 256, 2>(L, gsplit, st);
+        return run_variant<Op, 1, 32, 128, 4>(L, gsplit, st);
     case 5:
     case 6:
         if constexpr (!std::is_void<typename X2Of<Op>::type>::value) {

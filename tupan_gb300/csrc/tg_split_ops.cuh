@@ -7,6 +7,8 @@
 
 #pragma once
 
+#include <type_traits>
+
 #include "tg_common.cuh"
 
 namespace tg {
@@ -266,29 +268,38 @@ __device__ __forceinline__ void kahan_add2(float2 &sum, float2 &corr,
 struct PosI2 { float2 nxh, nyh, nzh, nxl, nyl, nzl, e2; };
 struct PosVelI2 { float2 nxh, nyh, nzh, nxl, nyl, nzl, e2, nvx, nvy, nvz; };
 
-// rsqrt with one Newton step on both lanes: y (3/2 - s y^2 / 2), masked to 0
-// where s == h2 (r2 == 0: self pairs and coincident particles).
-__device__ __forceinline__ float2 rsqrt_nr2(float2 s, float2 h2)
+// Forms of 1/sqrt in the packed operators: the MUFU approximation, a Newton
+// step y (3/2 - s y^2 / 2), or the Newton step of the scalar operators
+// (rsqrt_nr, operation for operation; one more than the other).
+enum PackedRsq : int { RSQ_RAW = 0, RSQ_NEWTON = 1, RSQ_SCALAR = 2 };
+
+template <int NR>
+__device__ __forceinline__ float2 rsq2_unmasked(float2 s)
 {
-    float2 y = make_float2(rsqrtf(s.x), rsqrtf(s.y));
-    float2 u = mul2(mul2(s, y), y);
-    y = mul2(y, fma2(u, dup(-0.5f), dup(1.5f)));
-    y.x = (s.x > h2.x) ? y.x : 0.0f;
-    y.y = (s.y > h2.y) ? y.y : 0.0f;
+    const float2 y = make_float2(rsqrtf(s.x), rsqrtf(s.y));
+    if constexpr (NR == RSQ_NEWTON) {
+        const float2 u = mul2(mul2(s, y), y);
+        return mul2(y, fma2(u, dup(-0.5f), dup(1.5f)));
+    }
+    if constexpr (NR == RSQ_SCALAR) {
+        const float2 t = mul2(s, y);
+        const float2 e = fma2(t, make_float2(-y.x, -y.y), dup(1.0f));
+        return fma2(mul2(y, dup(0.5f)), e, y);
+    }
     return y;
 }
 
-template <bool NR>
+// Masked to 0 where s == h2 (r2 == 0: self pairs and coincident particles).
+template <int NR>
 __device__ __forceinline__ float2 rsq2(float2 s, float2 h2)
 {
-    if constexpr (NR) return rsqrt_nr2(s, h2);
-    float2 y = make_float2(rsqrtf(s.x), rsqrtf(s.y));
+    float2 y = rsq2_unmasked<NR>(s);
     y.x = (s.x > h2.x) ? y.x : 0.0f;
     y.y = (s.y > h2.y) ? y.y : 0.0f;
     return y;
 }
 
-template <bool NR>
+template <int NR>
 struct PhiS2N {
     using P = PhiS::P;
     using I = PosI2;
@@ -318,7 +329,7 @@ struct PhiS2N {
     }
 };
 
-template <bool NR>
+template <int NR>
 struct AccS2N {
     using P = PhiS::P;
     using I = PosI2;
@@ -343,7 +354,7 @@ struct AccS2N {
     }
 };
 
-template <bool NR>
+template <int NR>
 struct AccJerkS2N {
     using P = AccJerkS::P;
     using I = PosVelI2;
@@ -389,21 +400,7 @@ struct PosVelMI2 {
     float2 nxh, nyh, nzh, nxl, nyl, nzl, e2, nvx, nvy, nvz, m;
 };
 
-__device__ __forceinline__ float2 rsqrt_nr2_raw(float2 s)
-{
-    float2 y = make_float2(rsqrtf(s.x), rsqrtf(s.y));
-    float2 u = mul2(mul2(s, y), y);
-    return mul2(y, fma2(u, dup(-0.5f), dup(1.5f)));
-}
-
-template <bool NR>
-__device__ __forceinline__ float2 rsq2_unmasked(float2 s)
-{
-    if constexpr (NR) return rsqrt_nr2_raw(s);
-    return make_float2(rsqrtf(s.x), rsqrtf(s.y));
-}
-
-template <bool NR>
+template <int NR>
 struct TstepS2N {
     static constexpr bool HAS_H2 = false;
     using P = AccJerkS::P;
@@ -450,7 +447,7 @@ struct SnapI2 {
         njx, njy, njz;
 };
 
-template <bool NR>
+template <int NR>
 struct SnapS2N {
     static constexpr bool HAS_H2 = false;
     using P = SnapS::P;
@@ -532,5 +529,18 @@ template <bool NR> struct X2Of<AccSN<NR>> { using type = AccS2N<NR>; };
 template <bool NR> struct X2Of<AccJerkSN<NR>> { using type = AccJerkS2N<NR>; };
 template <bool NR> struct X2Of<TstepSN<NR>> { using type = TstepS2N<NR>; };
 template <bool NR> struct X2Of<SnapSN<NR>> { using type = SnapS2N<NR>; };
+
+// A scalar Newton operator evaluated in packed pairs with its own bits: the
+// scalar 1/sqrt, and a tile's tail summed as one run like the scalar loop.
+template <class Op> struct Paired : Op {};
+template <> struct X2Of<Paired<PhiS>> { using type = PhiS2N<RSQ_SCALAR>; };
+template <> struct X2Of<Paired<AccS>> { using type = AccS2N<RSQ_SCALAR>; };
+template <> struct X2Of<Paired<AccJerkS>> {
+    using type = AccJerkS2N<RSQ_SCALAR>;
+};
+template <> struct X2Of<Paired<TstepS>> { using type = TstepS2N<RSQ_SCALAR>; };
+template <> struct X2Of<Paired<SnapS>> { using type = SnapS2N<RSQ_SCALAR>; };
+template <class Op> struct IsPaired : std::false_type {};
+template <class Op> struct IsPaired<Paired<Op>> : std::true_type {};
 
 }  // namespace tg
