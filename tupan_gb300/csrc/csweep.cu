@@ -139,9 +139,14 @@ __device__ __forceinline__ float ct_round_grid(double v, int e)
 }
 
 // box[0..2]: ordered minima, box[3..5]: ordered maxima (initialised to
-// 0xffffffff and 0 by the host).
-__global__ void ct_bbox(const double *x, const double *y, const double *z,
-                        uint64_t n, uint32_t *box)
+// 0xffffffff and 0 by the host).  Atomics to the six words serialise, so a
+// block reduces its own box first and BOX_BLOCKS blocks at most take part.
+constexpr int BOX_THREADS = 256;
+constexpr int BOX_BLOCKS = 304;       // two a multiprocessor
+
+__global__ void __launch_bounds__(BOX_THREADS)
+ct_bbox(const double *x, const double *y, const double *z, uint64_t n,
+        uint32_t *box)
 {
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
     float hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
@@ -161,12 +166,24 @@ __global__ void ct_bbox(const double *x, const double *y, const double *z,
             lo[d] = fminf(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], off));
             hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], off));
         }
+    __shared__ float wlo[BOX_THREADS / 32][3], whi[BOX_THREADS / 32][3];
     if ((threadIdx.x & 31) == 0)
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            atomicMin(&box[d], ord_of(lo[d]));
-            atomicMax(&box[3 + d], ord_of(hi[d]));
+            wlo[threadIdx.x >> 5][d] = lo[d];
+            whi[threadIdx.x >> 5][d] = hi[d];
         }
+    __syncthreads();
+    if (threadIdx.x < 3) {
+        const int d = threadIdx.x;
+        float l = wlo[0][d], h = whi[0][d];
+        for (int w = 1; w < BOX_THREADS / 32; ++w) {
+            l = fminf(l, wlo[w][d]);
+            h = fmaxf(h, whi[w][d]);
+        }
+        atomicMin(&box[d], ord_of(l));
+        atomicMax(&box[3 + d], ord_of(h));
+    }
 }
 
 __device__ __forceinline__ uint64_t spread3(uint32_t v)
@@ -211,90 +228,126 @@ __global__ void ct_keys(const double *x, const double *y, const double *z,
 
 // ---------------------------------------------------------------------------
 // Stable LSD radix sort of (48-bit key, 32-bit value) pairs, 8 bits a pass:
-// per-block digit counts, one exclusive scan over (digit, block), then a
-// stable scatter (warp-level ranks by __match_any_sync, warps in order).
+// per-block digit counts, then a stable scatter (warp-level ranks by
+// __match_any_sync, warps in order) whose blocks each sum the counts they
+// need themselves.
+//
+// Latency bounds a pass (12 bytes a key in and out are 0.5 us at N = 262144).
+// One CTA that scanned all (digit, block) counts between the two kernels
+// took 9 us of a pass's 27 at N = 65536 and 52 of 70 at 262144; RS_BLOCKS
+// blocks that read the 128 KiB of counts from L2 instead cost about 2, and a
+// pass takes 11 and 14.  As many blocks at every n above RS_BLOCKS * RS_THREADS
+// keys: fewer leave multiprocessors idle, more read more counts each.  Whole
+// sweeps against the scan: Acc 1.46 -> 1.40 ms at N = 46400, 33.7 -> 33.4 ms
+// at 262144 (with ct_bbox's reduction by blocks, 36 -> 6 us there).
 // ---------------------------------------------------------------------------
-constexpr int RS_THREADS = 256;
-constexpr int RS_ROUNDS = 8;
-constexpr int RS_TILE = RS_THREADS * RS_ROUNDS;
+constexpr int RS_THREADS = 512;
+constexpr uint32_t RS_BLOCKS = 128;
 constexpr int RS_PASSES = 6;
+constexpr uint32_t RS_DIGITS = 256;
 
-__global__ void __launch_bounds__(RS_THREADS)
-rs_count(const uint64_t *key, uint32_t n, int shift, uint32_t *counts)
+// Rounds of RS_THREADS keys that one block takes, and the blocks of n keys.
+__host__ __device__ constexpr uint32_t rs_rounds(uint32_t n)
 {
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
+    const uint64_t per = (uint64_t)RS_THREADS * RS_BLOCKS;
+    return (uint32_t)((n + per - 1) / per);
+}
+
+__host__ __device__ constexpr uint32_t rs_blocks(uint32_t n)
+{
+    const uint64_t tile = (uint64_t)rs_rounds(n) * RS_THREADS;
+    return (uint32_t)((n + tile - 1) / tile);
+}
+
+// counts[block][digit]
+__global__ void __launch_bounds__(RS_THREADS)
+rs_count(const uint64_t *key, uint32_t n, int rounds, int shift,
+         uint32_t *counts)
+{
+    __shared__ uint32_t h[RS_DIGITS];
+    if (threadIdx.x < RS_DIGITS) h[threadIdx.x] = 0;
     __syncthreads();
-    const uint32_t base = blockIdx.x * RS_TILE;
-    for (int r = 0; r < RS_ROUNDS; ++r) {
-        const uint32_t i = base + r * RS_THREADS + threadIdx.x;
+    const uint64_t base = (uint64_t)blockIdx.x * rounds * RS_THREADS;
+#pragma unroll 4
+    for (int r = 0; r < rounds; ++r) {
+        const uint64_t i = base + (uint64_t)r * RS_THREADS + threadIdx.x;
         if (i < n) atomicAdd(&h[(uint32_t)(key[i] >> shift) & 255u], 1u);
     }
     __syncthreads();
-    counts[threadIdx.x * gridDim.x + blockIdx.x] = h[threadIdx.x];
-}
-
-// Exclusive scan in place of `total` counts, one CTA of 1024 threads.
-__global__ void __launch_bounds__(1024)
-rs_scan(uint32_t *counts, uint32_t total)
-{
-    __shared__ uint32_t wsum[32];
-    const uint32_t t = threadIdx.x;
-    const uint32_t chunk = (total + 1023) / 1024;
-    const uint32_t b = t * chunk;
-    const uint32_t e = b + chunk < total ? b + chunk : total;
-    uint32_t s = 0;
-    for (uint32_t i = b; i < e; ++i) s += counts[i];
-    uint32_t incl = s;
-#pragma unroll
-    for (int off = 1; off < 32; off <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
-        if ((t & 31) >= (uint32_t)off) incl += v;
-    }
-    if ((t & 31) == 31) wsum[t >> 5] = incl;
-    __syncthreads();
-    if (t < 32) {
-        uint32_t w = wsum[t], wi = w;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, wi, off);
-            if (t >= (uint32_t)off) wi += v;
-        }
-        wsum[t] = wi - w;
-    }
-    __syncthreads();
-    uint32_t run = wsum[t >> 5] + incl - s;
-    for (uint32_t i = b; i < e; ++i) {
-        const uint32_t c = counts[i];
-        counts[i] = run;
-        run += c;
-    }
+    if (threadIdx.x < RS_DIGITS)
+        counts[blockIdx.x * RS_DIGITS + threadIdx.x] = h[threadIdx.x];
 }
 
 __global__ void __launch_bounds__(RS_THREADS)
 rs_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
-           uint32_t *vout, uint32_t n, int shift, const uint32_t *offs)
+           uint32_t *vout, uint32_t n, int rounds, int shift,
+           const uint32_t *counts)
 {
     constexpr int NW = RS_THREADS / 32;
-    __shared__ uint32_t base_d[256];
-    __shared__ uint32_t wcnt[NW][256];
+    constexpr int ROWS = RS_THREADS / (RS_DIGITS / 4);  // rows a step
+    static_assert(NW * RS_DIGITS >= 2 * ROWS * RS_DIGITS, "sums fit in wcnt");
+    __shared__ uint32_t base_d[RS_DIGITS];
+    __shared__ uint32_t wtot[RS_DIGITS / 32];
+    __shared__ __align__(16) uint32_t wcnt[NW][RS_DIGITS];
     const int t = threadIdx.x, w = t >> 5, lane = t & 31;
-    base_d[t] = offs[t * gridDim.x + blockIdx.x];
+
+    // First place of each digit of this block: the counts of lower digits
+    // in all blocks and of this digit in earlier ones.  A thread sums four
+    // digits over every ROWS-th block.
+    {
+        const uint4 *row = (const uint4 *)counts + (t & 63);
+        uint4 all = make_uint4(0, 0, 0, 0), low = all;
+#pragma unroll 8
+        for (uint32_t b = t >> 6; b < gridDim.x; b += ROWS) {
+            const uint4 c = row[b * (RS_DIGITS / 4)];
+            const uint32_t m = b < blockIdx.x ? 0xffffffffu : 0u;
+            all.x += c.x; all.y += c.y; all.z += c.z; all.w += c.w;
+            low.x += c.x & m; low.y += c.y & m;
+            low.z += c.z & m; low.w += c.w & m;
+        }
+        ((uint4 *)wcnt)[t] = all;
+        ((uint4 *)wcnt)[RS_THREADS + t] = low;
+    }
+    __syncthreads();
+    uint32_t tot = 0, before = 0, incl = 0;
+    if (t < (int)RS_DIGITS) {
+        const uint32_t *sums = &wcnt[0][0];
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            tot += sums[r * RS_DIGITS + t];
+            before += sums[(ROWS + r) * RS_DIGITS + t];
+        }
+        incl = tot;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += v;
+        }
+        if (lane == 31) wtot[w] = incl;
+    }
+    __syncthreads();
+    if (t < (int)RS_DIGITS) {
+        uint32_t run = incl - tot + before;
+        for (int q = 0; q < w; ++q) run += wtot[q];
+        base_d[t] = run;
+    }
+
     const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t base = blockIdx.x * RS_TILE;
-    for (int r = 0; r < RS_ROUNDS; ++r) {
-        for (int d = lane; d < 256; d += 32) wcnt[w][d] = 0;
-        __syncthreads();
-        const uint32_t i = base + r * RS_THREADS + t;
+    const uint64_t base = (uint64_t)blockIdx.x * rounds * RS_THREADS;
+    for (int r = 0; r < rounds; ++r) {
+        const uint64_t i = base + (uint64_t)r * RS_THREADS + t;
         const bool ok = i < n;
         const uint64_t k = ok ? kin[i] : 0;
         const uint32_t v = ok ? vin[i] : 0;
+#pragma unroll
+        for (int d = lane; d < (int)RS_DIGITS; d += 32) wcnt[w][d] = 0;
+        __syncwarp();
         const uint32_t dg = ok ? ((uint32_t)(k >> shift) & 255u) : 256u;
         const uint32_t peers = __match_any_sync(0xffffffffu, dg);
         const uint32_t rank = __popc(peers & lt);
         if (ok && rank == 0) wcnt[w][dg] = __popc(peers);
         __syncthreads();
-        {
+        if (t < (int)RS_DIGITS) {
             uint32_t run = base_d[t];
 #pragma unroll
             for (int q = 0; q < NW; ++q) {
@@ -310,26 +363,26 @@ rs_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
             kout[pos] = k;
             vout[pos] = v;
         }
-        __syncthreads();
-    }
+        __syncwarp();       // a warp's own counters are read before the next
+    }                       // round clears them
 }
 
 // Sorts n (key, val) pairs; the result ends in (ka, va) (an even number of
-// passes); kb, vb are scratch of n entries, counts 256 x ceil(n / RS_TILE).
+// passes); kb, vb are scratch of n entries, counts rs_blocks(n) x 256.
 static cudaError_t radix_sort(uint64_t *ka, uint32_t *va, uint64_t *kb,
                               uint32_t *vb, uint32_t *counts, uint32_t n,
                               cudaStream_t st)
 {
-    const uint32_t nb = (n + RS_TILE - 1) / RS_TILE;
+    const uint32_t nb = rs_blocks(n);
+    const int rounds = (int)rs_rounds(n);
     for (int p = 0; p < RS_PASSES; ++p) {
         const int shift = 8 * p;
         uint64_t *ki = (p & 1) ? kb : ka, *ko = (p & 1) ? ka : kb;
         uint32_t *vi = (p & 1) ? vb : va, *vo = (p & 1) ? va : vb;
-        rs_count<<<nb, RS_THREADS, 0, st>>>(ki, n, shift, counts);
-        rs_scan<<<1, 1024, 0, st>>>(counts, 256u * nb);
-        rs_scatter<<<nb, RS_THREADS, 0, st>>>(ki, vi, ko, vo, n, shift,
-                                              counts);
-        g_launch_count += 3;
+        rs_count<<<nb, RS_THREADS, 0, st>>>(ki, n, rounds, shift, counts);
+        rs_scatter<<<nb, RS_THREADS, 0, st>>>(ki, vi, ko, vo, n, rounds,
+                                              shift, counts);
+        g_launch_count += 2;
     }
     return cudaGetLastError();
 }
@@ -924,17 +977,18 @@ static CtLayout ct_layout(int k, uint64_t ni, uint64_t nj, bool same,
 {
     const uint64_t nmax = ni > nj ? ni : nj;
     const uint64_t ntiles = (nj + CT - 1) / CT;
-    const uint64_t nb = (nmax + RS_TILE - 1) / RS_TILE;
     CtLayout L;
     size_t o = 0;
     L.box = o;     o += 256;
     L.key_a = o;   o += up256(8 * nmax);
     L.key_b = o;   o += up256(8 * nmax);
     L.val_b = o;   o += up256(4 * nmax);
-    L.counts = o;  o += up256(4 * 256 * nb);
     L.perm_i = o;  o += up256(4 * ni);
     L.perm_j = same ? L.perm_i : o;
     if (!same) o += up256(4 * nj);
+    // The sorts' counts (1 KiB a block, a block 512 keys or more) may run on
+    // into the records and tiles, which are written after the sorts.
+    L.counts = o;  o += 1024 * ((nmax + 2047) / 2048);
     L.irec = o;    o += up256(48 * ni);
     L.tiles = o;   o += up256(4 * ntiles * (uint64_t)ct_block_floats(k));
     L.partial = o;
@@ -1008,6 +1062,12 @@ static cudaError_t ct_run(const CtLaunch &L, int gsplit, cudaStream_t st)
     return cudaGetLastError();
 }
 
+static unsigned box_grid(uint64_t n)
+{
+    const uint64_t b = (n + BOX_THREADS - 1) / BOX_THREADS;
+    return (unsigned)(b < BOX_BLOCKS ? b : BOX_BLOCKS);
+}
+
 static unsigned grid_for(uint64_t n)
 {
     uint64_t b = (n + 255) / 256;
@@ -1053,10 +1113,10 @@ cudaError_t launch_centred(int k, uint64_t ni, const void *const *ia,
     // bounding box of both sets, Morton order of each
     TG_CUDA_TRY(cudaMemsetAsync(box, 0xff, 3 * sizeof(uint32_t), st));
     TG_CUDA_TRY(cudaMemsetAsync(box + 3, 0, 3 * sizeof(uint32_t), st));
-    ct_bbox<<<grid_for(ni), 256, 0, st>>>(AI.a[1], AI.a[2], AI.a[3], ni, box);
+    ct_bbox<<<box_grid(ni), BOX_THREADS, 0, st>>>(AI.a[1], AI.a[2], AI.a[3], ni, box);
     g_launch_count += 1;
     if (!same && nj) {
-        ct_bbox<<<grid_for(nj), 256, 0, st>>>(AJ.a[1], AJ.a[2], AJ.a[3], nj,
+        ct_bbox<<<box_grid(nj), BOX_THREADS, 0, st>>>(AJ.a[1], AJ.a[2], AJ.a[3], nj,
                                               box);
         g_launch_count += 1;
     }
