@@ -77,4 +77,14 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar,
     return false;
 }
 
+// Adds one to a counter in shared memory and returns its old value: what the
+// warps that came before did is visible to the last, and may be overwritten.
+__device__ __forceinline__ uint32_t arrive_acq_rel(uint32_t *count)
+{
+    uint32_t old;
+    asm volatile("atom.acq_rel.cta.shared::cta.add.u32 %0, [%1], 1;"
+                 : "=r"(old) : "r"(smem_u32(count)) : "memory");
+    return old;
+}
+
 }  // namespace tg
