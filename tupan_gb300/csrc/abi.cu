@@ -47,8 +47,10 @@ namespace tg {
 template <typename R>
 cudaError_t launch_exact(const Sweep &s, cudaStream_t st, long long budget,
                          unsigned *err);
-cudaError_t launch_pack(int kernel, uint64_t n, const void *const *attrs,
-                        float4 *out, cudaStream_t st);
+cudaError_t launch_pack_both(int kernel, uint64_t ni, const unsigned *ni_dev,
+                             const void *const *iattrs, float4 *iout,
+                             uint64_t nj, const void *const *jattrs,
+                             float4 *jout, cudaStream_t st);
 cudaError_t launch_split(int kernel, const float4 *irec, const float4 *jrec,
                          uint64_t ni, uint64_t nj, void *const *out,
                          double *partial, int variant, int gsplit, double eta,
@@ -352,12 +354,9 @@ int run_device_sweep(DeviceState *d, Sweep &s, cudaStream_t st)
     if (rc) return rc;
     float4 *irec = (float4 *)d->pack;
     float4 *jrec = same ? irec : (float4 *)((char *)d->pack + ibytes);
-    e = launch_pack(k, s.ni, s.ip, irec, st);
+    e = launch_pack_both(k, s.ni, nullptr, s.ip, irec, same ? 0 : s.nj, s.jp,
+                         jrec, st);
     if (e != cudaSuccess) return cuda_fail(e, "pack launch");
-    if (!same) {
-        e = launch_pack(k, s.nj, s.jp, jrec, st);
-        if (e != cudaSuccess) return cuda_fail(e, "pack launch");
-    }
     if (gsplit > 1) {
         rc = grow((void **)&d->partial, &d->partial_bytes,
                   (size_t)gsplit * n_out(k) * s.ni * sizeof(double),

@@ -45,15 +45,14 @@ namespace tg {
 template <typename R>
 cudaError_t launch_exact(const Sweep &s, cudaStream_t st, long long budget,
                          unsigned *err);
-cudaError_t launch_pack(int kernel, uint64_t n, const void *const *attrs,
-                        float4 *out, cudaStream_t st);
 cudaError_t launch_split(int kernel, const float4 *irec, const float4 *jrec,
                          uint64_t ni, uint64_t nj, void *const *out,
                          double *partial, int variant, int gsplit, double eta,
                          unsigned *err, cudaStream_t st);
-cudaError_t launch_pack_dev(int kernel, uint64_t n, const unsigned *n_dev,
-                            const void *const *attrs, float4 *out,
-                            cudaStream_t st);
+cudaError_t launch_pack_both(int kernel, uint64_t ni, const unsigned *ni_dev,
+                             const void *const *iattrs, float4 *iout,
+                             uint64_t nj, const void *const *jattrs,
+                             float4 *jout, cudaStream_t st);
 cudaError_t launch_split_dev(int kernel, const float4 *irec,
                              const float4 *jrec, uint64_t ni,
                              const unsigned *ni_dev, uint64_t nj,
@@ -407,9 +406,9 @@ cudaError_t bsweep(Block *b, int kernel, uint64_t ni, const double *const *ia,
     s.ni_dev = b->count_dev;
     if (b->mode == MODE_EXACT)
         return launch_exact<double>(s, b->stream, 1LL << 20, b->err);
-    cudaError_t e = launch_pack_dev(kernel, ni, b->count_dev, s.ip, b->pack_i,
-                                    b->stream);
-    if (e == cudaSuccess) e = launch_pack(kernel, b->n, s.jp, b->pack_j, b->stream);
+    cudaError_t e = launch_pack_both(kernel, ni, b->count_dev, s.ip,
+                                     b->pack_i, b->n, s.jp, b->pack_j,
+                                     b->stream);
     if (e != cudaSuccess) return e;
     int variant, gsplit;
     choose_split_public(kernel, ni, b->n, &variant, &gsplit);

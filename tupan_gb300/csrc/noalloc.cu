@@ -35,8 +35,10 @@
 #define TG_EXPORT extern "C" __attribute__((visibility("default")))
 
 namespace tg {
-cudaError_t launch_pack(int kernel, uint64_t n, const void *const *attrs,
-                        float4 *out, cudaStream_t st);
+cudaError_t launch_pack_both(int kernel, uint64_t ni, const unsigned *ni_dev,
+                             const void *const *iattrs, float4 *iout,
+                             uint64_t nj, const void *const *jattrs,
+                             float4 *jout, cudaStream_t st);
 cudaError_t launch_split(int kernel, const float4 *irec, const float4 *jrec,
                          uint64_t ni, uint64_t nj, void *const *out,
                          double *partial, int variant, int gsplit, double eta,
@@ -193,8 +195,9 @@ TG_EXPORT int tupan_gb300_acc_jerk_split_noalloc(
     void *out[6] = {iax, iay, iaz, ijx, ijy, ijz};
     const int gsplit = pick_gsplit(ni, nj, g_sms[dev]);
     cudaError_t e = cudaMemsetAsync(g_err_ptr[dev], 0, sizeof(unsigned), st);
-    if (e == cudaSuccess) e = launch_pack(K_ACC_JERK, ni, ia, irec, st);
-    if (e == cudaSuccess) e = launch_pack(K_ACC_JERK, nj, ja, jrec, st);
+    if (e == cudaSuccess)
+        e = launch_pack_both(K_ACC_JERK, ni, nullptr, ia, irec, nj, ja, jrec,
+                             st);
     if (e == cudaSuccess)
         e = launch_split(K_ACC_JERK, irec, jrec, ni, nj, out,
                          g_partial_ptr[dev], NOALLOC_VARIANT, gsplit, 0.0,

@@ -36,8 +36,10 @@
 
 namespace tg {
 
-cudaError_t launch_pack(int kernel, uint64_t n, const void *const *attrs,
-                        float4 *out, cudaStream_t st);
+cudaError_t launch_pack_both(int kernel, uint64_t ni, const unsigned *ni_dev,
+                             const void *const *iattrs, float4 *iout,
+                             uint64_t nj, const void *const *jattrs,
+                             float4 *jout, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Learned start: parameters in device memory.
@@ -746,10 +748,9 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
                 return ST_CUDA;
             g_work.rec_cap = need;
         }
-        if (launch_pack(K_ACC_JERK, ni, i_attrs, g_work.rec, st) != cudaSuccess)
-            return ST_CUDA;
-        if (!same && launch_pack(K_ACC_JERK, nj, j_attrs, g_work.rec + ni * 3,
-                                 st) != cudaSuccess)
+        if (launch_pack_both(K_ACC_JERK, ni, nullptr, i_attrs, g_work.rec,
+                             same ? 0 : nj, j_attrs, g_work.rec + ni * 3,
+                             st) != cudaSuccess)
             return ST_CUDA;
         irec = g_work.rec;
         jrec = same ? g_work.rec : g_work.rec + ni * 3;

@@ -42,8 +42,10 @@ namespace tg {
 template <typename R>
 cudaError_t launch_exact(const Sweep &s, cudaStream_t st, long long budget,
                          unsigned *err);
-cudaError_t launch_pack(int kernel, uint64_t n, const void *const *attrs,
-                        float4 *out, cudaStream_t st);
+cudaError_t launch_pack_both(int kernel, uint64_t ni, const unsigned *ni_dev,
+                             const void *const *iattrs, float4 *iout,
+                             uint64_t nj, const void *const *jattrs,
+                             float4 *jout, cudaStream_t st);
 cudaError_t launch_split(int kernel, const float4 *irec, const float4 *jrec,
                          uint64_t ni, uint64_t nj, void *const *out,
                          double *partial, int variant, int gsplit, double eta,
@@ -701,8 +703,8 @@ cudaError_t sweep(Sia *S, int kernel, uint64_t ilo, uint64_t ni, uint64_t jlo,
     const int nf = split_nf_host(kernel);
     float4 *irec = (float4 *)S->pack;
     float4 *jrec = irec + ni * nf;
-    cudaError_t e = launch_pack(kernel, ni, s.ip, irec, S->stream);
-    if (e == cudaSuccess) e = launch_pack(kernel, nj, s.jp, jrec, S->stream);
+    cudaError_t e = launch_pack_both(kernel, ni, nullptr, s.ip, irec, nj,
+                                     s.jp, jrec, S->stream);
     if (e != cudaSuccess) return e;
     int variant, gsplit;
     choose_split_public(kernel, ni, nj, &variant, &gsplit);
