@@ -26,6 +26,7 @@
 #include <unordered_map>
 
 #include "tg_common.cuh"
+#include "tg_launch.cuh"
 
 #if defined(TG_ABI_FLOAT64)
 typedef double REAL;
@@ -79,6 +80,7 @@ cudaError_t launch_centred(int k, uint64_t ni, const void *const *ia,
 
 namespace tg {
 std::atomic<unsigned long long> g_launch_count{0};
+thread_local bool g_chain_capture = false;
 std::atomic<uint32_t> g_pipe_spin{1u << 20};
 uint32_t pipe_spin_limit() { return g_pipe_spin.load(); }
 std::atomic<float> g_centred_mid{3.0f};

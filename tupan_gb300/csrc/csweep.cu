@@ -48,6 +48,7 @@
 #include <type_traits>
 
 #include "tg_common.cuh"
+#include "tg_launch.cuh"
 #include "tg_split_ops.cuh"
 #include "tg_tma.cuh"
 
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(BOX_THREADS)
 ct_bbox(const double *x, const double *y, const double *z, uint64_t n,
         uint32_t *box)
 {
+    chain_begin();
     float lo[3] = {FLT_MAX, FLT_MAX, FLT_MAX};
     float hi[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX};
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -203,6 +205,7 @@ __global__ void ct_keys(const double *x, const double *y, const double *z,
                         uint64_t n, const uint32_t *box, uint64_t *key,
                         uint32_t *val)
 {
+    chain_begin();
     double lo[3], ext = 0.0;
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -264,6 +267,7 @@ __global__ void __launch_bounds__(RS_THREADS)
 rs_count(const uint64_t *key, uint32_t n, int rounds, int shift,
          uint32_t *counts)
 {
+    chain_begin();
     __shared__ uint32_t h[RS_DIGITS];
     if (threadIdx.x < RS_DIGITS) h[threadIdx.x] = 0;
     __syncthreads();
@@ -283,6 +287,7 @@ rs_scatter(const uint64_t *kin, const uint32_t *vin, uint64_t *kout,
            uint32_t *vout, uint32_t n, int rounds, int shift,
            const uint32_t *counts)
 {
+    chain_begin();
     constexpr int NW = RS_THREADS / 32;
     constexpr int ROWS = RS_THREADS / (RS_DIGITS / 4);  // rows a step
     static_assert(NW * RS_DIGITS >= 2 * ROWS * RS_DIGITS, "sums fit in wcnt");
@@ -379,12 +384,13 @@ static cudaError_t radix_sort(uint64_t *ka, uint32_t *va, uint64_t *kb,
         const int shift = 8 * p;
         uint64_t *ki = (p & 1) ? kb : ka, *ko = (p & 1) ? ka : kb;
         uint32_t *vi = (p & 1) ? vb : va, *vo = (p & 1) ? va : vb;
-        rs_count<<<nb, RS_THREADS, 0, st>>>(ki, n, rounds, shift, counts);
-        rs_scatter<<<nb, RS_THREADS, 0, st>>>(ki, vi, ko, vo, n, rounds,
-                                              shift, counts);
+        TG_CUDA_TRY(launch_chained(rs_count, nb, RS_THREADS, 0, st, ki, n,
+                                   rounds, shift, counts));
+        TG_CUDA_TRY(launch_chained(rs_scatter, nb, RS_THREADS, 0, st, ki, vi,
+                                   ko, vo, n, rounds, shift, counts));
         g_launch_count += 2;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 // ---------------------------------------------------------------------------
@@ -403,6 +409,7 @@ __global__ void __launch_bounds__(CT)
 ct_tiles(const CtAttrs A, uint64_t nj, const uint32_t *perm,
          const uint32_t *box, float *tiles)
 {
+    chain_begin();
     constexpr int NF = ct_nf(K), TB = ct_block_floats(K);
     __shared__ double red[6][CT / 32];
     __shared__ float redf[CT / 32];
@@ -491,6 +498,7 @@ template <int K>
 __global__ void ct_pack_i(const CtAttrs A, uint64_t ni, const uint32_t *perm,
                           float4 *irec)
 {
+    chain_begin();
     for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < ni;
          s += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t o = perm[s];
@@ -659,6 +667,7 @@ constexpr size_t ct_smem_bytes()
 template <class Op, int NI, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) ct_sweep(const CtLaunch L)
 {
+    chain_begin();
     constexpr int NO = Op::NO, K = Op::K;
     constexpr int TB = ct_block_floats(K);
     static_assert((TB * 4) % 16 == 0, "tile blocks must stay 16-byte aligned");
@@ -956,6 +965,7 @@ template <int NO>
 __global__ void __launch_bounds__(128)
 ct_finalize(const CtLaunch L, int gsplit)
 {
+    chain_begin();
     // one thread an (i, output), eight loads in flight before their
     // additions
     constexpr int RUN = 8;
@@ -1066,17 +1076,16 @@ static cudaError_t ct_run(const CtLaunch &L, int gsplit, cudaStream_t st)
             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         attr.store(1);
     }
-    ct_sweep<Op, NI, NT, MINB><<<dim3((unsigned)gx, (unsigned)gsplit), NT,
-                                 smem, st>>>(L);
+    cudaError_t e = launch_chained(ct_sweep<Op, NI, NT, MINB>,
+                                   dim3((unsigned)gx, (unsigned)gsplit), NT,
+                                   smem, st, L);
     g_launch_count += 1;
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || gsplit == 1) return e;
     uint64_t blocks = (L.ni + 127) / 128;
     if (blocks > 152 * 8) blocks = 152 * 8;
-    ct_finalize<Op::NO><<<dim3((unsigned)blocks, Op::NO), 128, 0, st>>>(
-        L, gsplit);
     g_launch_count += 1;
-    return cudaGetLastError();
+    return launch_chained(ct_finalize<Op::NO>, dim3((unsigned)blocks, Op::NO),
+                          128, 0, st, L, gsplit);
 }
 
 static unsigned box_grid(uint64_t n)
@@ -1130,48 +1139,38 @@ cudaError_t launch_centred(int k, uint64_t ni, const void *const *ia,
     // bounding box of both sets, Morton order of each
     TG_CUDA_TRY(cudaMemsetAsync(box, 0xff, 3 * sizeof(uint32_t), st));
     TG_CUDA_TRY(cudaMemsetAsync(box + 3, 0, 3 * sizeof(uint32_t), st));
-    ct_bbox<<<box_grid(ni), BOX_THREADS, 0, st>>>(AI.a[1], AI.a[2], AI.a[3], ni, box);
+    TG_CUDA_TRY(launch_chained(ct_bbox, box_grid(ni), BOX_THREADS, 0, st,
+                               AI.a[1], AI.a[2], AI.a[3], ni, box));
     g_launch_count += 1;
     if (!same && nj) {
-        ct_bbox<<<box_grid(nj), BOX_THREADS, 0, st>>>(AJ.a[1], AJ.a[2], AJ.a[3], nj,
-                                              box);
+        TG_CUDA_TRY(launch_chained(ct_bbox, box_grid(nj), BOX_THREADS, 0, st,
+                                   AJ.a[1], AJ.a[2], AJ.a[3], nj, box));
         g_launch_count += 1;
     }
-    ct_keys<<<grid_for(ni), 256, 0, st>>>(AI.a[1], AI.a[2], AI.a[3], ni, box,
-                                          ka, perm_i);
+    TG_CUDA_TRY(launch_chained(ct_keys, grid_for(ni), 256, 0, st, AI.a[1],
+                               AI.a[2], AI.a[3], ni, box, ka, perm_i));
     g_launch_count += 1;
     TG_CUDA_TRY(radix_sort(ka, perm_i, kb, vb, counts, (uint32_t)ni, st));
     if (!same && nj) {
-        ct_keys<<<grid_for(nj), 256, 0, st>>>(AJ.a[1], AJ.a[2], AJ.a[3], nj,
-                                              box, ka, perm_j);
+        TG_CUDA_TRY(launch_chained(ct_keys, grid_for(nj), 256, 0, st, AJ.a[1],
+                                   AJ.a[2], AJ.a[3], nj, box, ka, perm_j));
         g_launch_count += 1;
         TG_CUDA_TRY(radix_sort(ka, perm_j, kb, vb, counts, (uint32_t)nj, st));
     }
 
     // tiles and i-records
     if (ntiles) {
-        switch (k) {
-        case K_PHI:
-            ct_tiles<K_PHI><<<(unsigned)ntiles, CT, 0, st>>>(AJ, nj, perm_j, box,
-                                                    tiles);
-            break;
-        case K_ACC:
-            ct_tiles<K_ACC><<<(unsigned)ntiles, CT, 0, st>>>(AJ, nj, perm_j, box,
-                                                    tiles);
-            break;
-        default:
-            ct_tiles<K_ACC_JERK><<<(unsigned)ntiles, CT, 0, st>>>(AJ, nj, perm_j, box,
-                                                    tiles);
-            break;
-        }
+        auto *tile = k == K_PHI   ? ct_tiles<K_PHI>
+                     : k == K_ACC ? ct_tiles<K_ACC>
+                                  : ct_tiles<K_ACC_JERK>;
+        TG_CUDA_TRY(launch_chained(tile, (unsigned)ntiles, CT, 0, st, AJ, nj,
+                                   perm_j, box, tiles));
         g_launch_count += 1;
     }
-    if (k == K_ACC_JERK)
-        ct_pack_i<K_ACC_JERK><<<grid_for(ni), 256, 0, st>>>(AI, ni, perm_i, irec);
-    else
-        ct_pack_i<K_ACC><<<grid_for(ni), 256, 0, st>>>(AI, ni, perm_i, irec);
+    auto *pack = k == K_ACC_JERK ? ct_pack_i<K_ACC_JERK> : ct_pack_i<K_ACC>;
+    TG_CUDA_TRY(launch_chained(pack, grid_for(ni), 256, 0, st, AI, ni, perm_i,
+                               irec));
     g_launch_count += 1;
-    TG_CUDA_TRY(cudaGetLastError());
 
     CtLaunch L;
     memset(&L, 0, sizeof(L));

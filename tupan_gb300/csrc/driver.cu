@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "tg_common.cuh"
+#include "tg_launch.cuh"
 #include "tg_pairs.cuh"
 
 #define TG_EXPORT extern "C" __attribute__((visibility("default")))
@@ -101,6 +102,7 @@ constexpr int STAGE_T = 64;
 // itself whether the end time is reached.
 __global__ void k_begin_step(Arrays A, uint64_t n, StepCtl *c)
 {
+    chain_begin();
     const bool done = fabs(c->t) >= c->t_end;
     const int d = blockIdx.y;
     if (threadIdx.x == 0 && blockIdx.x == 0 && d == 0) {
@@ -120,6 +122,7 @@ __global__ void k_begin_step(Arrays A, uint64_t n, StepCtl *c)
 // the last block through turns it into the step.
 __global__ void k_min_tstep(const double *x, uint64_t n, StepCtl *c)
 {
+    chain_begin();
     if (c->done) return;
     unsigned long long best = 0x7ff0000000000000ull;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -150,6 +153,7 @@ __global__ void k_min_tstep(const double *x, uint64_t n, StepCtl *c)
 template <int ORDER>
 __global__ void k_predict(Arrays A, uint64_t n, const StepCtl *c)
 {
+    chain_begin();
     if (c->done) return;
     const double tau = c->tau;
     const int d = blockIdx.y;
@@ -190,6 +194,7 @@ template <int ORDER>
 __global__ void k_correct(Arrays A, uint64_t n, StepCtl *c, bool last,
                           double *tau_log, long long cap)
 {
+    chain_begin();
     if (c->done) return;
     const double tau = c->tau;
     const int d = blockIdx.y;
@@ -364,22 +369,28 @@ cudaError_t step_order(Hermite *h)
     const unsigned b = grid_for(h->n, h->sms);
     const dim3 g(b, 3);
     cudaStream_t st = h->stream;
-    k_begin_step<<<g, STAGE_T, 0, st>>>(h->A, h->n, h->ctl);
+    cudaError_t e = launch_chained(k_begin_step, g, STAGE_T, 0, st, h->A, h->n,
+                                   h->ctl);
+    if (e != cudaSuccess) return e;
     if (h->adaptive) {
         const double *at[8] = {h->A.m, h->A.r[0], h->A.r[1], h->A.r[2],
                                h->A.e2, h->A.v[0], h->A.v[1], h->A.v[2]};
-        cudaError_t e = sweep(h, K_TSTEP, at, h->A.dt, h->eta);
+        e = sweep(h, K_TSTEP, at, h->A.dt, h->eta);
         if (e != cudaSuccess) return e;
-        k_min_tstep<<<b, STAGE_T, 0, st>>>(h->A.dt[0], h->n, h->ctl);
+        e = launch_chained(k_min_tstep, b, STAGE_T, 0, st, h->A.dt[0], h->n,
+                           h->ctl);
+        if (e != cudaSuccess) return e;
     }
-    cudaError_t e = forces(h, h->A.r0, h->A.v0, h->A.f0);
+    e = forces(h, h->A.r0, h->A.v0, h->A.f0);
     if (e != cudaSuccess) return e;
-    k_predict<ORDER><<<g, STAGE_T, 0, st>>>(h->A, h->n, h->ctl);
+    e = launch_chained(k_predict<ORDER>, g, STAGE_T, 0, st, h->A, h->n, h->ctl);
+    if (e != cudaSuccess) return e;
     for (int pass = 0; pass < 2; ++pass) {
         e = forces(h, h->A.r, h->A.v, h->A.f1);
         if (e != cudaSuccess) return e;
-        k_correct<ORDER><<<g, STAGE_T, 0, st>>>(h->A, h->n, h->ctl, pass == 1,
-                                                h->tau_log, h->tau_cap);
+        e = launch_chained(k_correct<ORDER>, g, STAGE_T, 0, st, h->A, h->n,
+                           h->ctl, pass == 1, h->tau_log, h->tau_cap);
+        if (e != cudaSuccess) return e;
     }
     g_launch_count += h->adaptive ? 5 : 4;
     return cudaGetLastError();
@@ -504,7 +515,9 @@ TG_EXPORT int tupan_gb300_hermite_evolve(void *handle, double t_end,
             cudaSuccess)
             return ST_CUDA;
         cudaError_t e = cudaSuccess;
+        g_chain_capture = true;
         for (int k = 0; k < batch && e == cudaSuccess; ++k) e = one_step(h);
+        g_chain_capture = false;
         cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
         if (e != cudaSuccess || e2 != cudaSuccess) return ST_CUDA;
         if (cudaGraphInstantiate(&h->graph, g, 0) != cudaSuccess) return ST_CUDA;

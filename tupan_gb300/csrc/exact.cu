@@ -9,6 +9,7 @@
 // accuracy of CUDA's transcendental functions.
 
 #include "tg_common.cuh"
+#include "tg_launch.cuh"
 #include "tg_kepler.cuh"
 #include "tg_ordered.cuh"
 #include "tg_pairs.cuh"
@@ -46,6 +47,7 @@ exact_terms(const Sweep s, const int li)
     constexpr int LP = P == 1 ? 0 : P == 2 ? 1 : 2;
     static_assert(P == 1 << LP, "P is 1, 2 or 4");
     __shared__ __align__(16) R buf[2][NO][T * P];
+    chain_begin();
     const uint64_t ni = s.ni_dev ? (uint64_t)*s.ni_dev : s.ni, nj = s.nj;
     const uint64_t i0 = (uint64_t)blockIdx.x << li;
     // blocks past a device-side count have no i (the whole block leaves)
@@ -161,6 +163,7 @@ exact_few(const Sweep s)
     constexpr int RUNS = FEW_T / ORD_RUN, SPAN = ORD_PITCH * ORD_K;
     constexpr int ROW = RUNS * SPAN + 1;      // odd: outputs on other banks
     __shared__ double buf[2][NO][ROW];
+    chain_begin();
     const uint64_t i = blockIdx.x, nj = s.nj;
     if (s.ni_dev && i >= (uint64_t)*s.ni_dev) return;
     const int tid = threadIdx.x, lane = tid & 31;
@@ -291,9 +294,9 @@ static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
         // equal, 1000 x 1000 137 against 107).
         constexpr uint64_t most = few_owned<Op>() == Op::NO ? 5000 : 2 * 152;
         if (s.ni <= most) {
-            exact_few<Op><<<(unsigned)s.ni, few_threads<Op>(), 0, st>>>(s);
             g_launch_count += 1;
-            return cudaGetLastError();
+            return launch_chained(exact_few<Op>, (unsigned)s.ni,
+                                  few_threads<Op>(), 0, st, s);
         }
     }
     // As many i a block as leave 600 blocks (four an SM): more i share a j
@@ -304,9 +307,9 @@ static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
     while ((Op::NO << li) > T) --li;
     while ((1 << li) > P && (s.ni >> li) < 600) --li;
     const unsigned blocks = (unsigned)((s.ni + (1u << li) - 1) >> li);
-    exact_terms<Op, R, T, P, BLK><<<blocks, T, 0, st>>>(s, li);
     g_launch_count += 1;
-    return cudaGetLastError();
+    return launch_chained(exact_terms<Op, R, T, P, BLK>, blocks, T, 0, st, s,
+                          li);
 }
 
 template <typename R>

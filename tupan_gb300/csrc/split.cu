@@ -25,6 +25,7 @@
 #include <type_traits>
 
 #include "tg_common.cuh"
+#include "tg_launch.cuh"
 #include "tg_pn.cuh"
 #include "tg_split_ops.cuh"
 #include "tg_tma.cuh"
@@ -148,6 +149,7 @@ template <int NF>
 __global__ void __launch_bounds__(PACK_T)
 pack_records(const PackSet s0, const PackSet s1)
 {
+    chain_begin();
     const bool second = blockIdx.x >= s0.blocks;
     const PackSet &p = second ? s1 : s0;
     const uint64_t b = second ? blockIdx.x - s0.blocks : blockIdx.x;
@@ -197,14 +199,11 @@ cudaError_t launch_pack_both(int kernel, uint64_t ni, const unsigned *ni_dev,
     if (ni == 0 && nj == 0) return cudaSuccess;
     const PackSet a = pack_set(kernel, ni, ni_dev, iattrs, iout);
     const PackSet b = pack_set(kernel, nj, nullptr, jattrs, jout);
-    const unsigned blocks = a.blocks + b.blocks;
-    switch (split_nf(kernel)) {
-    case 2: pack_records<2><<<blocks, PACK_T, 0, st>>>(a, b); break;
-    case 3: pack_records<3><<<blocks, PACK_T, 0, st>>>(a, b); break;
-    default: pack_records<5><<<blocks, PACK_T, 0, st>>>(a, b); break;
-    }
+    auto *pack = split_nf(kernel) == 2   ? pack_records<2>
+                 : split_nf(kernel) == 3 ? pack_records<3>
+                                         : pack_records<5>;
     g_launch_count += 1;
-    return cudaGetLastError();
+    return launch_chained(pack, a.blocks + b.blocks, PACK_T, 0, st, a, b);
 }
 
 cudaError_t launch_pack(int kernel, uint64_t n, const void *const *attrs,
@@ -258,6 +257,7 @@ split_sweep(const SplitLaunch L)
     const int tid = threadIdx.x;
     const int js = tid % JS;
     const int grp = tid / JS;
+    chain_begin();
     const uint64_t ni = L.ni_dev ? (uint64_t)*L.ni_dev : L.ni;
     // CTAs past a device-side count have no i: the whole CTA leaves before
     // any barrier or copy exists
@@ -508,6 +508,7 @@ split_finalize(const SplitLaunch L, int gsplit)
 {
     constexpr int NO = Op::NO, MAXC = Op::MAXC, RUN = 8;
     __shared__ double part[FINALIZE_W][FINALIZE_I];
+    chain_begin();
     // a sweep CTA that reported an error left its partials unwritten
     if (*(volatile unsigned *)L.err) return;
     const uint64_t ni = L.ni_dev ? (uint64_t)*L.ni_dev : L.ni;
@@ -616,16 +617,16 @@ static cudaError_t run_variant(const SplitLaunch &L, int gsplit,
     constexpr uint64_t IPC = (uint64_t)(NT / JS) * NI;
     const uint64_t gx = (L.ni + IPC - 1) / IPC;
     dim3 grid((unsigned)gx, (unsigned)gsplit);
-    split_sweep<Op, NI, JS, NT, MINB, X2><<<grid, NT, 0, st>>>(L);
+    cudaError_t e = launch_chained(split_sweep<Op, NI, JS, NT, MINB, X2>, grid,
+                                   NT, 0, st, L);
     g_launch_count += 1;
-    cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || gsplit == 1) return e;
     uint64_t blocks = (L.ni + FINALIZE_I - 1) / FINALIZE_I;
     if (blocks > 152 * 8) blocks = 152 * 8;
-    split_finalize<typename FinalOp<Op>::type><<<dim3((unsigned)blocks, Op::NO),
-                         dim3(FINALIZE_I, FINALIZE_W), 0, st>>>(L, gsplit);
     g_launch_count += 1;
-    return cudaGetLastError();
+    return launch_chained(split_finalize<typename FinalOp<Op>::type>,
+                          dim3((unsigned)blocks, Op::NO),
+                          dim3(FINALIZE_I, FINALIZE_W), 0, st, L, gsplit);
 }
 
 template <class Op>
