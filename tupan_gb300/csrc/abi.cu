@@ -475,7 +475,7 @@ int host_call(const HostCall &c)
     char *base = (char *)d->io;
     cudaError_t e;
     const size_t in_bytes = off[nh];
-    const bool pinned = total + sizeof(unsigned) <= PIN_MAX;
+    bool pinned = total + sizeof(unsigned) <= PIN_MAX;
     if (pinned && total + sizeof(unsigned) > d->pin_bytes) {
         // (outgrown at most a few times: sizes double up to PIN_MAX)
         if (d->pin) cudaFreeHost(d->pin);
@@ -483,9 +483,14 @@ int host_call(const HostCall &c)
         d->pin_bytes = 0;
         size_t want = 1 << 16;
         while (want < total + sizeof(unsigned)) want *= 2;
-        e = cudaHostAlloc((void **)&d->pin, want, cudaHostAllocDefault);
-        if (e != cudaSuccess) return cuda_fail(e, "pinned staging buffer");
-        d->pin_bytes = want;
+        if (cudaHostAlloc((void **)&d->pin, want, cudaHostAllocDefault) ==
+            cudaSuccess) {
+            d->pin_bytes = want;
+        } else {            // no memory to pin: copy from where the arrays are
+            cudaGetLastError();
+            d->pin = nullptr;
+            pinned = false;
+        }
     }
     if (pinned) {
         for (int h = 0; h < nh; ++h)
