@@ -592,7 +592,7 @@ split_sweep(const SplitLaunch L)
 // FP64 additions of 64 cycles.  A thread an i that added its six outputs
 // load by load, the form this replaces, took 117 us for 64 splits whatever
 // ni (16384 x 16384 AccJerk: 116 us after a 322 us sweep, 400 us in all;
-// now 347 us in all).
+// 347 us in all with this one, 341 with chained launches).
 constexpr int FINALIZE_I = 32, FINALIZE_W = 8;
 
 template <class Op>
