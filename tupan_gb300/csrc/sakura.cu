@@ -569,6 +569,14 @@ MlpParams g_mlp;
 bool g_have_mlp = false;
 int g_kepler_form = KEP_REFERENCE;   // tupan_gb300_kepler_set_form
 
+// Status of an allocation that failed.  The runtime's error is cleared: the
+// next sweep's launch would report it as its own.
+int out_of_memory()
+{
+    cudaGetLastError();
+    return ST_CUDA;
+}
+
 int grow_queue(size_t cap)
 {
     if (cap <= g_work.q_cap) return 0;
@@ -710,8 +718,10 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
     }
     if (ni > g_work.cnt_cap) {
         cudaFree(g_work.cnt);
+        g_work.cnt = nullptr;
+        g_work.cnt_cap = 0;
         if (cudaMalloc((void **)&g_work.cnt, ni * sizeof(unsigned)) != cudaSuccess)
-            return ST_CUDA;
+            return out_of_memory();
         g_work.cnt_cap = ni;
     }
     SakuraArgs A;
@@ -745,7 +755,7 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
             g_work.rec_cap = 0;
             if (cudaMalloc((void **)&g_work.rec, need * sizeof(float4)) !=
                 cudaSuccess)
-                return ST_CUDA;
+                return out_of_memory();
             g_work.rec_cap = need;
         }
         if (launch_pack_both(K_ACC_JERK, ni, nullptr, i_attrs, g_work.rec,
@@ -761,7 +771,7 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
     if (want > 1ull << 20) want = 1ull << 20;
     SakuraReport r;
     for (;;) {
-        if (grow_queue(want)) return ST_CUDA;
+        if (grow_queue(want)) return out_of_memory();
         A.queue_i = g_work.qi;
         A.queue_j = g_work.qj;
         A.queue_r = g_work.qr;
