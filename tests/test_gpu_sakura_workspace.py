@@ -1,5 +1,7 @@
 """The workspace that the queued Sakura sweep keeps between calls."""
 
+from concurrent.futures import ThreadPoolExecutor
+
 import numpy as np
 import pytest
 
@@ -48,3 +50,66 @@ def test_a_sweep_after_one_too_large_for_the_memory(mode):
                 np.testing.assert_array_equal(o.cpu().numpy(), w)
         else:
             assert all(np.isfinite(o.cpu().numpy()).all() for o in out)
+
+
+def test_systems_stepped_from_several_threads():
+    # sizes apart, so that the workspace grows under way; every system's bits
+    # are those of stepping it alone
+    sizes = (180, 700, 1201, 333)
+
+    def step(n, seed):
+        dev = kp.DeviceSakura(ics.plummer(n, eps=0.0, seed=seed,
+                                          masses="salpeter"))
+        got = []
+        for k in range(1, 9):
+            dev.evolve(1.0 / 256, k / 256.0)
+            got.append(dev.state())
+        dev.close()
+        return got
+
+    want = [step(n, n) for n in sizes]
+    with ThreadPoolExecutor(len(sizes)) as pool:
+        runs = [pool.submit(step, n, n) for n in sizes for _ in range(2)]
+        for k, r in enumerate(runs):
+            for a, b in zip(r.result(), want[k // 2]):
+                for c in a:
+                    np.testing.assert_array_equal(a[c], b[c])
+
+
+def test_sweeps_and_pair_solves_on_streams_of_several_threads():
+    torch = pytest.importorskip("torch")
+    sizes = (150, 900, 64, 2001)
+    sys_ = [system(n, n) for n in sizes]
+    rng = np.random.default_rng(3)
+    m = torch.from_numpy(rng.uniform(1e-4, 1e-2, 500)).cuda()
+    e2 = torch.zeros(500, dtype=torch.float64, device="cuda")
+    st = torch.from_numpy(rng.standard_normal((500, 6)) * 0.05).cuda()
+
+    def pairs(stream):
+        out = torch.zeros((500, 6), dtype=torch.float64, device="cuda")
+        torch.cuda.current_stream().synchronize()
+        kp.kepler_pairs(500, 1.0 / 512, m, e2, st, out, stream=stream)
+        return out.cpu().numpy()
+
+    want = []
+    for (d, out), n in zip(sys_, sizes):
+        for mode in ("exact", "split"):
+            nk = sweep(d, out, n, mode)
+            want.append((nk, [o.cpu().numpy() for o in out]))
+    want_pairs = pairs(None)
+    torch.cuda.synchronize()
+
+    def work(k):
+        (d, out), n = sys_[k], sizes[k]
+        s = torch.cuda.Stream()
+        for _ in range(6):
+            for q, mode in enumerate(("exact", "split")):
+                nk = sweep(d, out, n, mode, s.cuda_stream)
+                w = want[2 * k + q]
+                assert nk == w[0]
+                for o, x in zip(out, w[1]):
+                    np.testing.assert_array_equal(o.cpu().numpy(), x)
+            np.testing.assert_array_equal(pairs(s.cuda_stream), want_pairs)
+
+    with ThreadPoolExecutor(len(sizes)) as pool:
+        list(pool.map(work, range(len(sizes))))

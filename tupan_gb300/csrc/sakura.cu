@@ -28,6 +28,9 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <mutex>
+#include <unordered_map>
+
 #include "tg_common.cuh"
 #include "tg_kepler.cuh"
 #include "tg_split_ops.cuh"
@@ -551,7 +554,11 @@ using namespace tg;
 
 namespace {
 
+// Workspace of the queued sweeps and the pair solver on one device, grown as
+// needed.  A call holds `mu` until its stream has finished with it, so calls
+// from several threads or streams take turns.
 struct SakuraWork {
+    std::mutex mu;
     unsigned *cnt = nullptr;
     size_t cnt_cap = 0;
     unsigned *qi = nullptr, *qj = nullptr, *qr = nullptr;
@@ -564,35 +571,49 @@ struct SakuraWork {
     int sms = 0;
 };
 
-SakuraWork g_work;
 MlpParams g_mlp;
 bool g_have_mlp = false;
 int g_kepler_form = KEP_REFERENCE;   // tupan_gb300_kepler_set_form
 
-// Status of an allocation that failed.  The runtime's error is cleared: the
-// next sweep's launch would report it as its own.
-int out_of_memory()
+// The current device's workspace, or null without a device.
+SakuraWork *device_work()
 {
+    static std::mutex mu;
+    static std::unordered_map<int, SakuraWork *> works;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    std::lock_guard<std::mutex> lock(mu);
+    SakuraWork *&w = works[dev];
+    if (!w) w = new SakuraWork();
+    return w;
+}
+
+// Status of a call that failed part way: what it launched is waited for, as
+// the workspace goes to the next call, and the runtime's error is cleared,
+// which the next sweep's launch would report as its own.
+int failed(cudaStream_t st)
+{
+    cudaStreamSynchronize(st);
     cudaGetLastError();
     return ST_CUDA;
 }
 
-int grow_queue(size_t cap)
+int grow_queue(SakuraWork &W, size_t cap)
 {
-    if (cap <= g_work.q_cap) return 0;
-    cudaFree(g_work.qi);
-    cudaFree(g_work.qj);
-    cudaFree(g_work.qr);
-    cudaFree(g_work.contrib);
-    g_work.qi = g_work.qj = g_work.qr = nullptr;
-    g_work.contrib = nullptr;
-    g_work.q_cap = 0;
-    if (cudaMalloc((void **)&g_work.qi, cap * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc((void **)&g_work.qj, cap * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc((void **)&g_work.qr, cap * sizeof(unsigned)) != cudaSuccess ||
-        cudaMalloc((void **)&g_work.contrib, cap * 6 * sizeof(double)) != cudaSuccess)
+    if (cap <= W.q_cap) return 0;
+    cudaFree(W.qi);
+    cudaFree(W.qj);
+    cudaFree(W.qr);
+    cudaFree(W.contrib);
+    W.qi = W.qj = W.qr = nullptr;
+    W.contrib = nullptr;
+    W.q_cap = 0;
+    if (cudaMalloc((void **)&W.qi, cap * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc((void **)&W.qj, cap * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc((void **)&W.qr, cap * sizeof(unsigned)) != cudaSuccess ||
+        cudaMalloc((void **)&W.contrib, cap * 6 * sizeof(double)) != cudaSuccess)
         return 1;
-    g_work.q_cap = cap;
+    W.q_cap = cap;
     return 0;
 }
 
@@ -648,7 +669,8 @@ TG_EXPORT int tupan_gb300_kepler_set_form(int form)
 // Solves n independent pairs (DEVICE arrays: m, e2, state n x 6, out n x 6)
 // over dt with universal_kepler_solver's full retry logic; iters, rec_x
 // (n x 4) and rec_y (n) are optional.  use_mlp selects the learned start.
-// Synchronous; returns a status code (3: a solve hit the budget).
+// Synchronous, callable from several threads at once; returns a status code
+// (3: a solve hit the budget).
 TG_EXPORT int tupan_gb300_kepler_pairs(uint64_t n, double dt, const double *m,
                                        const double *e2, const double *state,
                                        double *out, int *iters, float *rec_x,
@@ -656,11 +678,15 @@ TG_EXPORT int tupan_gb300_kepler_pairs(uint64_t n, double dt, const double *m,
                                        long long budget, void *stream)
 {
     if (use_mlp && !g_have_mlp) return ST_BAD_ARGUMENT;
-    if (!g_work.err && cudaMalloc((void **)&g_work.err, sizeof(unsigned)) !=
-                           cudaSuccess)
-        return ST_CUDA;
     cudaStream_t st = (cudaStream_t)stream;
-    cudaMemsetAsync(g_work.err, 0, sizeof(unsigned), st);
+    SakuraWork *const work = device_work();
+    if (!work) return ST_CUDA;
+    SakuraWork &W = *work;
+    std::lock_guard<std::mutex> lock(W.mu);
+    if (!W.err &&
+        cudaMalloc((void **)&W.err, sizeof(unsigned)) != cudaSuccess)
+        return failed(st);
+    cudaMemsetAsync(W.err, 0, sizeof(unsigned), st);
     PairSolve P;
     memset(&P, 0, sizeof(P));
     P.n = n;
@@ -677,14 +703,14 @@ TG_EXPORT int tupan_gb300_kepler_pairs(uint64_t n, double dt, const double *m,
     P.form = g_kepler_form;
     P.mlp = g_mlp;
     if (n) {
-        k_pair_solve<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(P, g_work.err);
+        k_pair_solve<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(P, W.err);
         g_launch_count += 1;
     }
     unsigned h = 0;
-    if (cudaMemcpyAsync(&h, g_work.err, sizeof(unsigned),
-                        cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+    if (cudaMemcpyAsync(&h, W.err, sizeof(unsigned), cudaMemcpyDeviceToHost,
+                        st) != cudaSuccess ||
         cudaStreamSynchronize(st) != cudaSuccess)
-        return ST_CUDA;
+        return failed(st);
     return h ? ST_DEVICE : ST_OK;
 }
 
@@ -693,7 +719,8 @@ TG_EXPORT int tupan_gb300_kepler_pairs(uint64_t n, double dt, const double *m,
 // i_attrs/j_attrs: 8 device pointers each (m r e2 v); outs: 6.  Optional
 // iteration histogram: kepler_iters (host, 65 bins; bin k counts solves with
 // k Laguerre updates, the last bin k >= 64).  Returns the number of queued
-// (Kepler-branch) pairs in *n_kepler.  Synchronous.
+// (Kepler-branch) pairs in *n_kepler.  Synchronous, callable from several
+// threads and streams at once.
 TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
                                        uint64_t nj, const void *const *j_attrs,
                                        double dt, int64_t flag,
@@ -707,22 +734,25 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
     if (use_mlp && !g_have_mlp) return ST_BAD_ARGUMENT;
     if (ni == 0) return ST_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    if (!g_work.rep) {
+    SakuraWork *const work = device_work();
+    if (!work) return ST_CUDA;
+    SakuraWork &W = *work;
+    std::lock_guard<std::mutex> lock(W.mu);
+    if (!W.rep) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&g_work.sms, cudaDevAttrMultiProcessorCount,
+            cudaDeviceGetAttribute(&W.sms, cudaDevAttrMultiProcessorCount,
                                    dev) != cudaSuccess ||
-            cudaMalloc((void **)&g_work.rep, sizeof(SakuraReport)) !=
-                cudaSuccess)
-            return ST_CUDA;
+            cudaMalloc((void **)&W.rep, sizeof(SakuraReport)) != cudaSuccess)
+            return failed(st);
     }
-    if (ni > g_work.cnt_cap) {
-        cudaFree(g_work.cnt);
-        g_work.cnt = nullptr;
-        g_work.cnt_cap = 0;
-        if (cudaMalloc((void **)&g_work.cnt, ni * sizeof(unsigned)) != cudaSuccess)
-            return out_of_memory();
-        g_work.cnt_cap = ni;
+    if (ni > W.cnt_cap) {
+        cudaFree(W.cnt);
+        W.cnt = nullptr;
+        W.cnt_cap = 0;
+        if (cudaMalloc((void **)&W.cnt, ni * sizeof(unsigned)) != cudaSuccess)
+            return failed(st);
+        W.cnt_cap = ni;
     }
     SakuraArgs A;
     memset(&A, 0, sizeof(A));
@@ -735,12 +765,12 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
     for (int c = 0; c < 6; ++c) A.out[c] = (double *)outs[c];
     A.dt = dt;
     A.flag = flag;
-    A.cnt = g_work.cnt;
+    A.cnt = W.cnt;
     A.budget = budget > 0 ? budget : (1LL << 20);
     A.use_mlp = use_mlp;
     A.form = g_kepler_form;
     A.mlp = g_mlp;
-    A.rep = g_work.rep;
+    A.rep = W.rep;
     const unsigned blocks = (unsigned)((ni + SK_THREADS - 1) / SK_THREADS);
     const int li = sk_li(ni);
     const unsigned eblocks = (unsigned)((ni + (1u << li) - 1) >> li);
@@ -749,21 +779,21 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
         bool same = ni == nj;
         for (int a = 0; a < 8 && same; ++a) same = i_attrs[a] == j_attrs[a];
         const size_t need = (ni + (same ? 0 : nj)) * 3;
-        if (need > g_work.rec_cap) {
-            cudaFree(g_work.rec);
-            g_work.rec = nullptr;
-            g_work.rec_cap = 0;
-            if (cudaMalloc((void **)&g_work.rec, need * sizeof(float4)) !=
+        if (need > W.rec_cap) {
+            cudaFree(W.rec);
+            W.rec = nullptr;
+            W.rec_cap = 0;
+            if (cudaMalloc((void **)&W.rec, need * sizeof(float4)) !=
                 cudaSuccess)
-                return out_of_memory();
-            g_work.rec_cap = need;
+                return failed(st);
+            W.rec_cap = need;
         }
-        if (launch_pack_both(K_ACC_JERK, ni, nullptr, i_attrs, g_work.rec,
-                             same ? 0 : nj, j_attrs, g_work.rec + ni * 3,
+        if (launch_pack_both(K_ACC_JERK, ni, nullptr, i_attrs, W.rec,
+                             same ? 0 : nj, j_attrs, W.rec + ni * 3,
                              st) != cudaSuccess)
-            return ST_CUDA;
-        irec = g_work.rec;
-        jrec = same ? g_work.rec : g_work.rec + ni * 3;
+            return failed(st);
+        irec = W.rec;
+        jrec = same ? W.rec : W.rec + ni * 3;
     }
     // room for a pair in 32 (Salpeter spheres: 1 in 16 at N = 256, 125 at
     // 4096), at most 2^20 to begin with; the counts decide
@@ -771,27 +801,27 @@ TG_EXPORT int tupan_gb300_sakura_queue(uint64_t ni, const void *const *i_attrs,
     if (want > 1ull << 20) want = 1ull << 20;
     SakuraReport r;
     for (;;) {
-        if (grow_queue(want)) return out_of_memory();
-        A.queue_i = g_work.qi;
-        A.queue_j = g_work.qj;
-        A.queue_r = g_work.qr;
-        A.cap = g_work.q_cap;
-        A.contrib = g_work.contrib;
-        cudaMemsetAsync(g_work.rep, 0, sizeof(SakuraReport), st);
+        if (grow_queue(W, want)) return failed(st);
+        A.queue_i = W.qi;
+        A.queue_j = W.qj;
+        A.queue_r = W.qr;
+        A.cap = W.q_cap;
+        A.contrib = W.contrib;
+        cudaMemsetAsync(W.rep, 0, sizeof(SakuraReport), st);
         if (mode == MODE_SPLIT)
             k_sakura_split_pass<<<blocks, SK_THREADS, 0, st>>>(A, irec, jrec);
         else
             k_sakura_pass<<<eblocks, SK_THREADS, 0, st>>>(A, li);
-        k_scan<<<1, 1024, 0, st>>>(g_work.cnt, ni);
+        k_scan<<<1, 1024, 0, st>>>(W.cnt, ni);
         // the solves stride over the queue, whose length only the device
         // knows: five blocks of 96 registers a thread fill an SM
-        k_sakura_kepler<<<(unsigned)(5 * g_work.sms), SK_THREADS, 0, st>>>(A);
+        k_sakura_kepler<<<(unsigned)(5 * W.sms), SK_THREADS, 0, st>>>(A);
         k_sakura_gather<<<(unsigned)((ni + 3) / 4), SK_THREADS, 0, st>>>(A);
         g_launch_count += 4;
-        if (cudaMemcpyAsync(&r, g_work.rep, sizeof(r), cudaMemcpyDeviceToHost,
+        if (cudaMemcpyAsync(&r, W.rep, sizeof(r), cudaMemcpyDeviceToHost,
                             st) != cudaSuccess ||
             cudaStreamSynchronize(st) != cudaSuccess)
-            return ST_CUDA;
+            return failed(st);
         if (r.pairs <= A.cap) break;
         want = r.pairs + r.pairs / 4;
     }
