@@ -113,13 +113,15 @@ __device__ __forceinline__ bool positive(double r2)
     return b > 0 && b <= 0x7ff0000000000000ll;
 }
 
-// a > b for a, b not negative or NaN
+// a > b for b not negative, or either of them NaN (of any sign: 0 / 0 is one
+// with the sign set).  Unsigned, negative values and NaN lie above infinity.
 __device__ __forceinline__ bool greater(float a, float b) { return a > b; }
 
 __device__ __forceinline__ bool greater(double a, double b)
 {
-    const long long x = __double_as_longlong(a), y = __double_as_longlong(b);
-    return x > y && x <= 0x7ff0000000000000ll;
+    const unsigned long long x = (unsigned long long)__double_as_longlong(a),
+                             y = (unsigned long long)__double_as_longlong(b);
+    return x > y && x <= 0x7ff0000000000000ull;
 }
 
 __device__ __forceinline__ float larger(float a, float o) { return fmax(a, o); }
