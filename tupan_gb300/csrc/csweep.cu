@@ -676,6 +676,7 @@ __global__ void __launch_bounds__(NT, MINB) ct_sweep(const CtLaunch L)
     __shared__ __align__(8) uint64_t bar[CT_STAGES];
     __shared__ uint32_t done[CT_STAGES];   // warps that have used the stage
     __shared__ int last[CT_STAGES];        // its newest tile
+    __shared__ int gave_up;                // a warp has
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint64_t ibase =
@@ -691,6 +692,7 @@ __global__ void __launch_bounds__(NT, MINB) ct_sweep(const CtLaunch L)
             done[q] = 0;
             last[q] = -1;
         }
+        gave_up = 0;
         mbar_init_fence();
     }
     __syncthreads();
@@ -704,6 +706,26 @@ __global__ void __launch_bounds__(NT, MINB) ct_sweep(const CtLaunch L)
     };
     if (tid == 0)
         for (int q = 0; q < CT_STAGES && q < nt; ++q) issue(q);
+    // Whether tile t is in its stage.  The caller's limit bounds the copy: a
+    // warp may come to a stage that a slower warp has yet to leave, and goes
+    // on (to the full bound, or until a warp gives up) until the refill is
+    // issued, then tries `spin` times again.
+    auto arrived = [&](int t) {
+        uint64_t *b = &bar[t % CT_STAGES];
+        const uint32_t parity = (uint32_t)((t / CT_STAGES) & 1);
+        for (uint32_t k = 0; k < L.spin; ++k)
+            if (mbar_try_wait(b, parity)) return true;
+        const volatile int *newest = &last[t % CT_STAGES], *quit = &gave_up;
+        for (uint32_t k = 0;
+             k < MBAR_SPIN_LIMIT && *newest < t && !*quit; ++k)
+            if (mbar_try_wait(b, parity)) return true;
+        if (*newest >= t)
+            for (uint32_t k = 0; k < L.spin; ++k)
+                if (mbar_try_wait(b, parity)) return true;
+        *(volatile int *)&gave_up = 1;
+        atomicOr(L.err, (unsigned)DERR_PIPE_TIMEOUT);
+        return false;
+    };
 
     CtI ip[NI];
 #pragma unroll
@@ -839,10 +861,7 @@ __global__ void __launch_bounds__(NT, MINB) ct_sweep(const CtLaunch L)
     // AccJerk 64.25 -> 63.96; Phi at 65536 1.863 -> 1.813.
     bool ok = true;
     for (int t = 0; t < nt; ++t) {
-        const bool got = mbar_wait_bounded(&bar[t % CT_STAGES],
-                                           (uint32_t)((t / CT_STAGES) & 1),
-                                           L.err, L.spin);
-        if (!__all_sync(0xffffffffu, got)) {
+        if (!__all_sync(0xffffffffu, arrived(t))) {
             ok = false;
             break;
         }
@@ -929,7 +948,7 @@ __global__ void __launch_bounds__(NT, MINB) ct_sweep(const CtLaunch L)
         }
     }
     if (!__syncthreads_and(ok)) {
-        // A warp gave up (the others then find no refill and give up too):
+        // A warp gave up (the others then find no refill, and its word):
         // wait for the newest copy of each stage, which may still be in
         // flight, before the shared memory goes away, and leave without
         // writing results.
