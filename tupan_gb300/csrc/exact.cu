@@ -8,6 +8,8 @@
 // leapfrog branch is bit-identical, their Kepler branch agrees to the
 // accuracy of CUDA's transcendental functions.
 
+#include <type_traits>
+
 #include "tg_common.cuh"
 #include "tg_launch.cuh"
 #include "tg_kepler.cuh"
@@ -26,20 +28,21 @@ constexpr int EXACT_THREADS = 128;
 // no sum goes on to the next tile's pairs.
 //
 // Why: a sum's additions have to stay in order, the terms need not.  One i a
-// thread over all j (the form this replaces) put a 256-body sweep on two SMs
-// and a 3001-body one on 24, each at the latency of a chain of whole pairs;
-// here only the additions are a chain (64 cycles each in double) and any ni
-// fills the chip.  Bound: the FP64 pipe (20 additions of 19 SM cycles a
+// thread over all j (exact_sweep, the only form before) put a 256-body sweep
+// on two SMs and a 3001-body one on 24, each at the latency of a chain of
+// whole pairs; here only the additions are a chain (64 cycles each in double)
+// and any ni fills the chip.  Bound: the FP64 pipe (20 additions of 19 SM cycles a
 // warp of AccJerk pairs; ncu at N = 8192: 71 % of its peak, the integer pipe
 // that carries the products 57 %).  No j prefetch and 64 registers (eight
 // blocks of 128 an SM) beat a prefetch at four blocks by 10 %: the chains of
-// dependent additions want warps.  Measured, double, Phi / AccJerk /
-// SnapCrackle / Tstep: N = 256 268 / 533 / 1216 / 687 us before, 17 / 19 /
-// 27 / 25 us now; N = 3001 2.98 / 6.09 / 14.1 / 7.70 ms, now 0.32 / 0.53 /
-// 1.40 / 0.65 ms; N = 32768 61 / 128 / 302 / 157 ms, now 21 / 51 / 141 /
-// 54 ms.  float takes four i a thread (one load of a j for four pairs, one
-// 16-byte store of a term): Phi + Acc at N = 10007 2.3 ms before, 0.62 ms.
-template <class Op, typename R, int T, int P, int BLK>
+// dependent additions want warps.  Measured, double: AccJerk / SnapCrackle at
+// N = 3001 6.09 / 14.1 ms before, 0.53 / 1.40 ms now; Phi / AccJerk /
+// SnapCrackle / Tstep at N = 32768 61 / 128 / 302 / 157 ms, now 21 / 51 /
+// 141 / 54 ms.  float takes four i a thread (one load of a j for four pairs,
+// one 16-byte store of a term): Phi + Acc at N = 10007 2.3 ms before, 0.62.
+// SKIP: rows past the last j form no term (else one that nobody reads: the
+// branch costs 1 to 2 % of a long sweep).
+template <class Op, typename R, int T, int P, int BLK, bool SKIP>
 __global__ void __launch_bounds__(T, BLK)
 exact_terms(const Sweep s, const int li)
 {
@@ -79,7 +82,8 @@ exact_terms(const Sweep s, const int li)
 #pragma unroll
             for (int p = 0; p < P; ++p) {
                 R tp[NO];
-                Op::terms(ip[p], jp, tp, s, soft2[p]);
+                if (!SKIP || j0 + row < nj)
+                    Op::terms(ip[p], jp, tp, s, soft2[p]);
 #pragma unroll
                 for (int k = 0; k < NO; ++k) t[k][p] = tp[k];
             }
@@ -120,6 +124,7 @@ exact_terms(const Sweep s, const int li)
 // at one i a block: Phi 100 x 8192 387 -> 66 us, Tstep 576 -> 115, AccJerk
 // 447 -> 336, SnapCrackle 690 -> 405; NREG X at N = 256 33 -> 19 us.
 constexpr int FEW_T = 256;
+constexpr uint64_t FEW_I = 2 * 152;     // two blocks an SM
 
 template <class Op>
 __host__ __device__ constexpr bool few_own(int c)
@@ -180,9 +185,8 @@ exact_few(const Sweep s)
     const uint64_t tiles = (nj + FEW_T - 1) / FEW_T;
     for (uint64_t k = 0; k <= tiles; ++k) {
         if (forms) {
-            if (k < tiles) {
-                const uint64_t j = k * FEW_T + tid < nj ? k * FEW_T + tid
-                                                        : nj - 1;
+            const uint64_t j = k * FEW_T + tid;
+            if (j < nj) {
                 double jp[NA], t[NO];
 #pragma unroll
                 for (int a = 0; a < NA; ++a)
@@ -235,6 +239,73 @@ exact_few(const Sweep s)
     if (!own || lane == 0) ((double *)s.out[c])[i] = Op::finish(c, ip, o, s);
 }
 
+// One i a thread over all j, j through shared memory in tiles: against a
+// handful of j, which would leave most rows of a tile of exact_terms idle.
+// double, 70000 x 1 against exact_terms: AccJerk 6 us and 27, SnapCrackle 12
+// and 71.
+constexpr int SWEEP_T = 128;
+
+template <typename R> struct SakuraPair;
+
+// Whether exact_sweep takes a call.  The lines lie where it and exact_terms
+// take equally long.  double: one j always (SnapCrackle at 1000 20 us and 7), two but
+// against few i (SnapCrackle at 1000 20 and 13, Tstep at 20000 8 and 10),
+// three from 30000 i (SnapCrackle 34 and 21, Tstep 11 and 12; at 3000 Tstep
+// 8 and 10).  float: up to 8 j (equal at few i, SnapCrackle at 35000 11 and
+// 4).  Sakura, whose terms are solves: lanes of a warp that solve for
+// different i diverge, so the i have to be many (double x 1 at 3000 96 us
+// and 112, at 7000 142 and 124; x 3 at 20000 275 and 353, at 50000 589 and
+// 535; x 5 at 200000 3.14 and 2.80 ms).
+template <class Op, typename R>
+bool one_i_a_thread(uint64_t ni, uint64_t nj)
+{
+    constexpr bool solves = std::is_same<Op, SakuraPair<R>>::value;
+    if (solves && ((nj <= 1 && ni >= 6000) || (nj <= 3 && ni >= 32000) ||
+                   (nj <= 5 && ni >= 200000)))
+        return true;
+    if (sizeof(R) == 4) return !solves && nj <= 8;
+    return !solves && (nj <= 1 || (nj == 2 && ni > FEW_I) ||
+                       (nj == 3 && ni >= 30000));
+}
+
+template <class Op, typename R>
+__global__ void __launch_bounds__(SWEEP_T)
+exact_sweep(const Sweep s)
+{
+    constexpr int NA = Op::NA, NO = Op::NO;
+    __shared__ R tile[NA][SWEEP_T];
+    chain_begin();
+    const uint64_t ni = s.ni_dev ? (uint64_t)*s.ni_dev : s.ni, nj = s.nj;
+    // blocks past a device-side count have no i (the whole block leaves)
+    if ((uint64_t)blockIdx.x * SWEEP_T >= ni) return;
+    const uint64_t i = (uint64_t)blockIdx.x * SWEEP_T + threadIdx.x;
+    R ip[NA], jp[NA], o[NO];
+#pragma unroll
+    for (int a = 0; a < NA; ++a) ip[a] = ((const R *)s.ip[a])[i < ni ? i : ni - 1];
+#pragma unroll
+    for (int c = 0; c < NO; ++c) o[c] = R(0);
+    Softening<R> soft2;
+    if (nj) soft2.set(ip[4], ((const R *)s.jp[4])[0]);
+    for (uint64_t j0 = 0; j0 < nj; j0 += SWEEP_T) {
+        const int n = nj - j0 < SWEEP_T ? (int)(nj - j0) : SWEEP_T;
+        __syncthreads();
+        if ((int)threadIdx.x < n)
+#pragma unroll
+            for (int a = 0; a < NA; ++a)
+                tile[a][threadIdx.x] = ((const R *)s.jp[a])[j0 + threadIdx.x];
+        __syncthreads();
+        for (int jj = 0; jj < n; ++jj) {
+#pragma unroll
+            for (int a = 0; a < NA; ++a) jp[a] = tile[a][jj];
+            fold_pair<Op>(ip, jp, o, s, soft2);
+        }
+    }
+    if (i >= ni) return;
+#pragma unroll
+    for (int c = 0; c < NO; ++c)
+        ((R *)s.out[c])[i] = Op::finish(c, ip, o[c], s);
+}
+
 // sakura_kernel.c:33-62: Sigma_j (m_j/M)(two-body step - initial state).
 template <typename R>
 struct SakuraPair {
@@ -285,15 +356,22 @@ static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
     constexpr int T = EXACT_THREADS;
     constexpr int P = sizeof(R) == 8 ? 1 : Op::WIDE ? 1 : 4;
     constexpr int BLK = sizeof(R) == 8 ? (Op::WIDE ? 4 : 8) : 6;
+    if (one_i_a_thread<Op, R>(s.ni, s.nj)) {
+        const unsigned b = (unsigned)((s.ni + SWEEP_T - 1) / SWEEP_T);
+        g_launch_count += 1;
+        return launch_chained(exact_sweep<Op, R>, b, SWEEP_T, 0, st, s);
+    }
     if constexpr (sizeof(R) == 8) {
-        // One i a block where its sums are the bound: sums with warps of
-        // their own (Phi, Tstep) win up to 5000 i (Phi at 3001 x 3001 267 us
-        // against 320, at 8192 equal; Tstep at 5000 x 5000 1.61 against 1.81
-        // ms, at 8192 7 % slower), sums that share one while no SM has more
+        // One i a block where its sums are the bound: while no SM has more
         // than two blocks (AccJerk 300 x 8192 380 us against 477, 600 x 3000
-        // equal, 1000 x 1000 137 against 107).
-        constexpr uint64_t most = few_owned<Op>() == Op::NO ? 5000 : 2 * 152;
-        if (s.ni <= most) {
+        // equal, 1000 x 1000 137 against 107), and up to 5000 i if each sum
+        // has a warp of its own (Phi at 3001 x 3001 267 us against 320, at
+        // 8192 equal; Tstep at 5000 x 5000 1.61 against 1.81 ms, at 8192 7 %
+        // slower) and j enough to fill it (Phi at 1500 x 512 53 us against
+        // 41, x 1024 73 and 80; at 5000 x 1024 208 and 174, x 2048 318 and
+        // 345; Tstep at 5000 x 16 73 and 9).
+        constexpr uint64_t most = few_owned<Op>() == Op::NO ? 5000 : FEW_I;
+        if (s.ni <= FEW_I || (s.ni <= most && 3 * s.nj >= s.ni)) {
             g_launch_count += 1;
             return launch_chained(exact_few<Op>, (unsigned)s.ni,
                                   few_threads<Op>(), 0, st, s);
@@ -308,8 +386,17 @@ static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
     while ((1 << li) > P && (s.ni >> li) < 600) --li;
     const unsigned blocks = (unsigned)((s.ni + (1u << li) - 1) >> li);
     g_launch_count += 1;
-    return launch_chained(exact_terms<Op, R, T, P, BLK>, blocks, T, 0, st, s,
-                          li);
+    // A dear term is left out where nobody reads it: a Sakura solve (1000 x 4
+    // 246 us without, 97 with), and PnAcc's in double against fewer j than a
+    // tile may have rows (1000 x 4 46 us and 17; in a long sweep it would
+    // cost up to 13 %).
+    constexpr bool solves = std::is_same<Op, SakuraPair<R>>::value;
+    if constexpr (Op::WIDE && !solves && sizeof(R) == 8)
+        if (s.nj < T)
+            return launch_chained(exact_terms<Op, R, T, P, BLK, true>, blocks,
+                                  T, 0, st, s, li);
+    return launch_chained(exact_terms<Op, R, T, P, BLK, solves>, blocks, T, 0,
+                          st, s, li);
 }
 
 template <typename R>
