@@ -1,4 +1,5 @@
-"""EXACT sweeps either side of each line of the dispatch (few j, few i): the oracle's bits, and no shape far off the time of its neighbours."""
+"""EXACT sweeps either side of each line of the dispatch (few j, few i, many
+i): the oracle's bits, and no shape far off the time of its neighbours."""
 
 import ctypes
 
@@ -72,7 +73,9 @@ def test_double(kernel, ni, nj):
 
 
 FLOAT = ([(ni, nj) for ni in (1, 129) for nj in (1, 8, 9, 16, 17)] +
-         [(20000, 8), (20000, 9)])
+         [(20000, 33), (21000, 33), (33000, 9), (36001, 9), (36000, 9)] +
+         [(many + d, 130) for many in (33000, 40000, 42000, 64000)
+          for d in (-1, 0, 1)])
 
 
 @pytest.mark.parametrize("kernel", sorted(NIN))
@@ -104,3 +107,13 @@ def test_few_j_do_not_take_a_block_an_i(kernel, nj):
     pytest.importorskip("torch")
     assert (microseconds(kernel, 5000, nj, "float64") <
             2.0 * microseconds(kernel, 7000, nj, "float64"))
+
+
+@pytest.mark.parametrize("kernel", ["acc_kernel", "acc_jerk_kernel",
+                                    "snap_crackle_kernel"])
+def test_many_i_in_float_fill_the_chip(kernel):
+    # 3.7 times the i: with one i a thread 2.3 to 2.5 times as long, the
+    # lanes of the smaller sweep being idle in part
+    pytest.importorskip("torch")
+    assert (microseconds(kernel, 130000, 2048, "float32") <
+            2.75 * microseconds(kernel, 35000, 2048, "float32"))

@@ -239,31 +239,41 @@ exact_few(const Sweep s)
     if (!own || lane == 0) ((double *)s.out[c])[i] = Op::finish(c, ip, o, s);
 }
 
-// One i a thread over all j, j through shared memory in tiles: against a
-// handful of j, which would leave most rows of a tile of exact_terms idle.
-// double, 70000 x 1 against exact_terms: AccJerk 6 us and 27, SnapCrackle 12
-// and 71.
+// One i a thread over all j, j through shared memory in tiles: for many i,
+// where the threads fill the chip without the terms' way through shared
+// memory, in float, whose additions are cheap; and against a handful of j,
+// which would leave most rows of a tile of exact_terms idle.  Bound: issue
+// slots (float), the FP64 pipe.  float, 70000 x 16384 against exact_terms:
+// Acc 2.04 ms and 2.53, AccJerk 2.91 and 3.91, SnapCrackle 5.61 and 7.12;
+// double, 70000 x 1: AccJerk 6 us and 27, SnapCrackle 12 and 71.
 constexpr int SWEEP_T = 128;
 
 template <typename R> struct SakuraPair;
 
-// Whether exact_sweep takes a call.  The lines lie where it and exact_terms
-// take equally long.  double: one j always (SnapCrackle at 1000 20 us and 7), two but
+// Whether exact_sweep takes a call that exact_terms would serve with J rows a
+// tile.  The lines lie where the two take equally long, measured at 1 to
+// 16384 j.  double: one j always (SnapCrackle at 1000 20 us and 7), two but
 // against few i (SnapCrackle at 1000 20 and 13, Tstep at 20000 8 and 10),
 // three from 30000 i (SnapCrackle 34 and 21, Tstep 11 and 12; at 3000 Tstep
 // 8 and 10).  float: up to 8 j (equal at few i, SnapCrackle at 35000 11 and
-// 4).  Sakura, whose terms are solves: lanes of a warp that solve for
+// 4), else from MANY i (AccJerk x 16384 at 40000 2.35 and 2.37 ms, at 45000
+// 2.62 and 2.38), or from as many fewer as the tiles' empty rows make of them
+// (SnapCrackle at 35000 x 33, where exact_terms takes two tiles of 32, 18 us
+// and 9).  Sakura, whose terms are solves: lanes of a warp that solve for
 // different i diverge, so the i have to be many (double x 1 at 3000 96 us
 // and 112, at 7000 142 and 124; x 3 at 20000 275 and 353, at 50000 589 and
-// 535; x 5 at 200000 3.14 and 2.80 ms).
+// 535; x 5 at 200000 3.14 and 2.80 ms; float x 64 at 100000 640 and 624 us,
+// at 200000 1.30 and 1.15 ms).
 template <class Op, typename R>
-bool one_i_a_thread(uint64_t ni, uint64_t nj)
+bool one_i_a_thread(uint64_t ni, uint64_t nj, uint64_t J)
 {
     constexpr bool solves = std::is_same<Op, SakuraPair<R>>::value;
     if (solves && ((nj <= 1 && ni >= 6000) || (nj <= 3 && ni >= 32000) ||
                    (nj <= 5 && ni >= 200000)))
         return true;
-    if (sizeof(R) == 4) return !solves && nj <= 8;
+    if (sizeof(R) == 4)
+        return (!solves && nj <= 8) || (double)ni * ((nj + J - 1) / J * J) >=
+                                           (double)Op::MANY * nj;
     return !solves && (nj <= 1 || (nj == 2 && ni > FEW_I) ||
                        (nj == 3 && ni >= 30000));
 }
@@ -311,6 +321,7 @@ template <typename R>
 struct SakuraPair {
     static constexpr int NA = 8, NO = 6;
     static constexpr bool WIDE = true;
+    static constexpr uint64_t MANY = 150000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &s,
                                                  Softening<R> &)
@@ -356,7 +367,14 @@ static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
     constexpr int T = EXACT_THREADS;
     constexpr int P = sizeof(R) == 8 ? 1 : Op::WIDE ? 1 : 4;
     constexpr int BLK = sizeof(R) == 8 ? (Op::WIDE ? 4 : 8) : 6;
-    if (one_i_a_thread<Op, R>(s.ni, s.nj)) {
+    // As many i a block as leave 600 blocks (four an SM): more i share a j
+    // load and fill the warps that add, fewer leave SMs idle (AccJerk at
+    // N = 3001: 751 blocks of 4 i 0.55 ms, 376 of 8 i 0.70 ms; at 32768
+    // 8 or 16 i within 1 %).  The I x NO sums have to fit the block.
+    int li = 5;
+    while ((Op::NO << li) > T) --li;
+    while ((1 << li) > P && (s.ni >> li) < 600) --li;
+    if (one_i_a_thread<Op, R>(s.ni, s.nj, T * P >> li)) {
         const unsigned b = (unsigned)((s.ni + SWEEP_T - 1) / SWEEP_T);
         g_launch_count += 1;
         return launch_chained(exact_sweep<Op, R>, b, SWEEP_T, 0, st, s);
@@ -377,13 +395,6 @@ static cudaError_t run_exact(const Sweep &s, cudaStream_t st)
                                   few_threads<Op>(), 0, st, s);
         }
     }
-    // As many i a block as leave 600 blocks (four an SM): more i share a j
-    // load and fill the warps that add, fewer leave SMs idle (AccJerk at
-    // N = 3001: 751 blocks of 4 i 0.55 ms, 376 of 8 i 0.70 ms; at 32768
-    // 8 or 16 i within 1 %).  The I x NO sums have to fit the block.
-    int li = 5;
-    while ((Op::NO << li) > T) --li;
-    while ((1 << li) > P && (s.ni >> li) < 600) --li;
     const unsigned blocks = (unsigned)((s.ni + (1u << li) - 1) >> li);
     g_launch_count += 1;
     // A dear term is left out where nobody reads it: a Sakura solve (1000 x 4

@@ -190,7 +190,8 @@ __device__ __forceinline__ void inv_root(double r2, double h2, double *q,
 // how a term joins its sum (join: added, subtracted or the larger kept; sums
 // start from zero; fold does it), whether an output's terms nearly all have
 // one sign (one_signed: ordered_sum's fast case) and the last step of each
-// output (finish).  Terms of different j are independent, so they
+// output (finish).  MANY: the i from which a float sweep does best with one
+// i a thread.  Terms of different j are independent, so they
 // may be formed in any order; folding them in j order keeps the
 // reference's bits.
 enum Join : int { JOIN_ADD = 0, JOIN_SUB = 1, JOIN_MAX = 2 };
@@ -218,6 +219,7 @@ template <typename R>
 struct PhiPair {
     static constexpr int NA = 5, NO = 1;
     static constexpr bool WIDE = false;
+    static constexpr uint64_t MANY = 64000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &,
                                                  Softening<R> &soft2)
@@ -242,6 +244,7 @@ template <typename R>
 struct AccPair {
     static constexpr int NA = 5, NO = 3;
     static constexpr bool WIDE = false;
+    static constexpr uint64_t MANY = 42000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &,
                                                  Softening<R> &soft2)
@@ -272,6 +275,7 @@ template <typename R>
 struct AccJerkPair {
     static constexpr int NA = 8, NO = 6;
     static constexpr bool WIDE = false;
+    static constexpr uint64_t MANY = 42000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &,
                                                  Softening<R> &soft2)
@@ -314,6 +318,7 @@ template <typename R>
 struct SnapCracklePair {
     static constexpr int NA = 14, NO = 6;
     static constexpr bool WIDE = false;
+    static constexpr uint64_t MANY = 40000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &,
                                                  Softening<R> &soft2)
@@ -411,6 +416,7 @@ template <typename R>
 struct TstepPair {
     static constexpr int NA = 8, NO = 2;
     static constexpr bool WIDE = false;
+    static constexpr uint64_t MANY = 64000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &s,
                                                  Softening<R> &soft2)
@@ -463,6 +469,7 @@ template <typename R>
 struct NregXPair {
     static constexpr int NA = 8, NO = 7;
     static constexpr bool WIDE = false;
+    static constexpr uint64_t MANY = 33000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &s,
                                                  Softening<R> &soft2)
@@ -505,6 +512,7 @@ template <typename R>
 struct NregVPair {
     static constexpr int NA = 7, NO = 4;
     static constexpr bool WIDE = false;
+    static constexpr uint64_t MANY = 10000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &s,
                                                  Softening<R> &)

@@ -230,6 +230,7 @@ template <typename R>
 struct PnAccPair {
     static constexpr int NA = 8, NO = 3;
     static constexpr bool WIDE = true;    // keeps 128 registers a thread
+    static constexpr uint64_t MANY = 25000;
     __device__ __forceinline__ static void terms(const R *ip, const R *jp,
                                                  R *t, const Sweep &s,
                                                  Softening<R> &soft2)
