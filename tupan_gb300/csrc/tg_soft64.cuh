@@ -19,7 +19,8 @@
 // can be zero: no quotient or root of 53-bit significands is a 54-bit odd
 // one.  The correction needs |1 - x r| < 2^-21 and |1 - w t^2| < 2^-21.2;
 // over all 2^23 and 2^24 seeds, with the truncation of the operand, MUFU's
-// errors are at most 2^-22.4 (r) and 2^-22.5 (t).
+// errors are at most 2^-22.4 (r) and 2^-22.5 (t)
+// (tests/test_soft64_seed_bounds.py: every seed, and seeds at those limits).
 #pragma once
 
 #include <stdint.h>
