@@ -130,9 +130,12 @@ void set_error(int status, const char *fmt, ...)
     fprintf(stderr, "tupan_gb300: %s\n", g_message);
 }
 
+// (the runtime keeps the error until it is read: the next launch would report
+// it as its own)
 int cuda_fail(cudaError_t e, const char *what)
 {
     set_error(ST_CUDA, "%s: %s", what, cudaGetErrorString(e));
+    cudaGetLastError();
     return ST_CUDA;
 }
 
