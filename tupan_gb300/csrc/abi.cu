@@ -155,9 +155,10 @@ struct DeviceState {
     size_t pin_bytes = 0;
 };
 
-// Host-array calls whose arrays take at most this go through one pinned
-// buffer: the arrays are gathered into it and cross in one copy, the results
-// come back in another with the error word.  Fourteen copies of pageable
+// Host-array calls whose arrays, inputs and outputs each padded to 256 bytes,
+// take at most this go through one pinned buffer: the inputs are gathered
+// into it and cross in one copy, the results come back in another and the
+// error word in a third.  Fourteen copies of pageable
 // arrays cost about 5 us each: AccJerk of 256 bodies through the plugin took
 // 166 us a call, 92 with the buffer.  Larger arrays copy from where they are,
 // without the extra pass over them.
@@ -947,8 +948,8 @@ TG_EXPORT int tupan_gb300_sweep_plan(int kernel, uint64_t ni, uint64_t nj,
 }
 
 // Tries each main-loop wait of the pipelined sweeps (split, centred,
-// ensemble) makes on its copy barrier before it records DERR_PIPE_TIMEOUT
-// and the CTA leaves without writing results (default 2^20; 0 makes every
+// ensemble) makes on its copy barrier, once the copy is issued, before it
+// records DERR_PIPE_TIMEOUT and the CTA leaves without writing results (default 2^20; 0 makes every
 // such wait time out at once).  Returns the previous limit.
 TG_EXPORT unsigned tupan_gb300_set_pipe_spin_limit(unsigned limit)
 {

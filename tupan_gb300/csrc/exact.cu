@@ -1,5 +1,6 @@
 // EXACT-mode sweeps: the terms of the pairs are formed in parallel over i
-// and j and added to each i's sums in source order.  With the pair
+// and j (or by one thread an i, where that is the faster form) and added to
+// each i's sums in source order.  With the pair
 // arithmetic of tg_pairs.cuh and this file compiled with -fmad=false, every
 // output is bit-identical to the reference C kernel (tupan/lib/src/*.c) on
 // the same inputs, for REAL = double and REAL = float.
@@ -117,10 +118,13 @@ exact_terms(const Sweep s, const int li)
 // Few i against many j, double: one i a block, eight warps form the terms of
 // 256 j a tile while others sum the tile before.  A one-signed or max output
 // has a warp of its own (ordered_sum, or a maximum in any order); the others
-// share one, an output a lane, that adds term by term (their sums change
-// sign and binade too often for ordered_sum).  Bound: that chain of
+// share one, an output a lane, that adds term by term.  Bound: that chain of
 // additions, 64 cycles a term (AccJerk 100 x 8192 336 us, 273 of them the
-// chain), else the latency of a tile's pairs.  Measured against exact_terms
+// chain), else the latency of a tile's pairs.  ordered_sum and a warp each
+// for the signed outputs too, on terms of zero mean: slower to some thousand
+// j (AccJerk 100 x 1024 45 us and 73, x 8192 333 and 398; 3001 x 3001 529
+// and 1383), as their sums keep leaving their binade and six warps add where
+// one did, faster for long ones (x 65536 2.63 and 1.67 ms).  Measured against exact_terms
 // at one i a block: Phi 100 x 8192 387 -> 66 us, Tstep 576 -> 115, AccJerk
 // 447 -> 336, SnapCrackle 690 -> 405; NREG X at N = 256 33 -> 19 us.
 constexpr int FEW_T = 256;
